@@ -610,7 +610,11 @@ __device__ int decode_rotations_warp(const uint8_t* __restrict__ gray, const Fra
             }
         }
     }
-    alive = alive && (__ballot_sync(kFull, border_bad) & gmask) == 0;
+    // Every lane votes: the rotations of one quad can differ in `alive` when
+    // the contrast or a border sample lies at its limit within rounding, and a
+    // vote behind `alive &&` would leave the lanes of the others waiting.
+    const uint32_t bad_lanes = __ballot_sync(kFull, border_bad);
+    alive = alive && (bad_lanes & gmask) == 0;
     __syncwarp();
     if (alive) {
         for (int c = u; c < cells; c += 8) raw[c] = raw[c] - thresh;  // diff

@@ -3,9 +3,9 @@
 // gpu_detector.cu:1784-2254, generalised from one frame to a batch).
 //
 // Memory: one cudaMalloc per plan holds every per-frame buffer, carved at
-// 256-byte alignment; the per-frame state records and the result records
-// are each contiguous, so a batch costs one memset node and one result copy.
-// Detect calls never allocate.
+// 256-byte alignment; the per-frame state records are contiguous, so a batch
+// costs one memset node.  The result records are page-locked host memory that the
+// last kernel writes.  Detect calls never allocate.
 
 #include <cuda_runtime.h>
 
@@ -72,8 +72,9 @@ struct Plan::Impl {
     BatchDesc host_desc{};
     BatchDesc* dev_desc = nullptr;
     FrameIO* io_fixed = nullptr;     // device: arena frame buffers
-    FrameIO* io_caller = nullptr;    // device: caller pointers, device path
-    FrameIO* io_staging = nullptr;   // pinned
+    FrameIO* io_dev = nullptr;       // device: this launch's frames, written by its first kernel
+    FrameIO* io_staging = nullptr;   // pinned: caller pointers, device path
+    FrameIOArgs io_fixed_args{};     // arena frame buffers, as the first kernel's argument
     uint8_t* frames_dev = nullptr;
     uint8_t* frames_pinned = nullptr;
     size_t frame_bytes = 0;
@@ -83,13 +84,14 @@ struct Plan::Impl {
     WorkQueue* queue = nullptr;        // right after the states: one memset clears both
     size_t queue_bytes = 0;
     PersistParams persist;
-    uint8_t* results_dev = nullptr;
-    uint8_t* results_pinned = nullptr;
+    uint8_t* results_pinned = nullptr;  // written by the GPU
     size_t results_bytes = 0;
     size_t result_stride = 0;
     cudaGraphExec_t graph_host = nullptr;    // H2D of the staging buffer + pipeline + D2H
     cudaGraphExec_t graph_fixed = nullptr;   // pipeline + D2H on the plan's device frames
-    cudaGraphExec_t graph_device = nullptr;  // caller device frames
+    cudaGraphExec_t graph_device = nullptr;  // caller device frames (first kernel's argument)
+    cudaGraph_t graph_device_src = nullptr;  // holds stats_node
+    cudaGraphNode_t stats_node = nullptr;
     cudaStream_t user_stream = nullptr;      // caller stream for submits (null: own stream)
     LaunchConfig launch_cfg;
     int sm_count = 152;
@@ -118,43 +120,86 @@ struct Plan::Impl {
         if (io_staging) cudaFreeHost(io_staging);
     }
 
+    FrameIOArgs frame_args(int mode) const {
+        if (mode != 2) return io_fixed_args;
+        FrameIOArgs args{};
+        std::copy(io_staging, io_staging + host_desc.frames, args.f);
+        return args;
+    }
+
     // mode 0: staging H2D + pipeline on the plan's frames; 1: pipeline on
     // the plan's frames (inputs already copied); 2: caller device frames.
     void enqueue(int mode, cudaStream_t s, void* const* events = nullptr) {
         if (mode == 0) {
             cudaMemcpyAsync(frames_dev, frames_pinned, frame_bytes, cudaMemcpyHostToDevice, s);
-        } else if (mode == 2) {
-            cudaMemcpyAsync(io_caller, io_staging, sizeof(FrameIO) * host_desc.frames,
-                            cudaMemcpyHostToDevice, s);
         }
-        const FrameIO* io = mode == 2 ? io_caller : io_fixed;
         if (launch_cfg.persistent && !events) {
+            if (mode == 2) {
+                cudaMemcpyAsync(io_dev, io_staging, sizeof(FrameIO) * host_desc.frames,
+                                cudaMemcpyHostToDevice, s);
+            }
             cudaMemsetAsync(states, 0, states_bytes + queue_bytes, s);
-            enqueue_persistent(dev_desc, host_desc, io, queue, s, launch_cfg, sm_count, persist);
+            enqueue_persistent(dev_desc, host_desc, mode == 2 ? io_dev : io_fixed, queue, s, launch_cfg, sm_count,
+                               persist);
         } else {
             // Stage events (profile_device) always time the per-stage launches.
             cudaMemsetAsync(states, 0, states_bytes, s);
             const ForkJoin fork{branch, ev_fork, ev_join};
-            enqueue_pipeline(dev_desc, host_desc, io, s, launch_cfg, sm_count, branch ? &fork : nullptr,
-                             events);
+            enqueue_pipeline(dev_desc, host_desc, frame_args(mode), io_dev, s, launch_cfg, sm_count,
+                             branch ? &fork : nullptr, events);
         }
-        cudaMemcpyAsync(results_pinned, results_dev, results_bytes, cudaMemcpyDeviceToHost, s);
     }
 
     void launch(int mode, cudaStream_t s) {
-        cudaGraphExec_t g = mode == 0 ? graph_host : (mode == 1 ? graph_fixed : graph_device);
-        if (g) {
-            cudaGraphLaunch(g, s);
-        } else {
+        const cudaGraphExec_t g = mode == 0 ? graph_host : (mode == 1 ? graph_fixed : graph_device);
+        if (!g || (mode == 2 && !launch_cfg.persistent && !set_graph_frames())) {
             enqueue(mode, s);
+            return;
         }
+        cudaGraphLaunch(g, s);
+    }
+
+    // The caller's frames into the device-input graph.
+    bool set_graph_frames() {
+        const FrameIOArgs args = frame_args(2);
+        const BatchDesc* desc = dev_desc;
+        FrameIO* out = io_dev;
+        void* kernel_args[] = {&desc, const_cast<FrameIOArgs*>(&args), &out};
+        cudaKernelNodeParams p{};
+        p.func = const_cast<void*>(stats_kernel());
+        p.gridDim = dim3(host_desc.stats_ctas);
+        p.blockDim = dim3(256);
+        p.kernelParams = kernel_args;
+        if (cudaGraphExecKernelNodeSetParams(graph_device, stats_node, &p) == cudaSuccess) return true;
+        cudaGetLastError();
+        return false;
+    }
+
+    // The node of the first kernel in a captured device-input graph.
+    static cudaGraphNode_t find_stats_node(cudaGraph_t graph) {
+        size_t n = 0;
+        if (cudaGraphGetNodes(graph, nullptr, &n) != cudaSuccess) return nullptr;
+        std::vector<cudaGraphNode_t> nodes(n);
+        if (cudaGraphGetNodes(graph, nodes.data(), &n) != cudaSuccess) return nullptr;
+        for (cudaGraphNode_t node : nodes) {
+            cudaGraphNodeType type;
+            cudaKernelNodeParams p{};
+            if (cudaGraphNodeGetType(node, &type) == cudaSuccess && type == cudaGraphNodeTypeKernel &&
+                cudaGraphKernelNodeGetParams(node, &p) == cudaSuccess && p.func == stats_kernel()) {
+                return node;
+            }
+        }
+        return nullptr;
     }
 
     void destroy_graphs() {
         if (graph_host) cudaGraphExecDestroy(graph_host);
         if (graph_fixed) cudaGraphExecDestroy(graph_fixed);
         if (graph_device) cudaGraphExecDestroy(graph_device);
+        if (graph_device_src) cudaGraphDestroy(graph_device_src);
         graph_host = graph_fixed = graph_device = nullptr;
+        graph_device_src = nullptr;
+        stats_node = nullptr;
     }
 
     void capture_all() {
@@ -175,9 +220,23 @@ struct Plan::Impl {
             cudaGetLastError();
             return false;
         }
+        cudaGraphNode_t node = nullptr;
+        if (mode == 2 && !launch_cfg.persistent) {
+            node = find_stats_node(graph);
+            if (!node) {
+                cudaGetLastError();
+                cudaGraphDestroy(graph);
+                return false;  // direct launches
+            }
+        }
         cudaGraphExec_t exec = nullptr;
         const cudaError_t st = cudaGraphInstantiate(&exec, graph, 0);
-        cudaGraphDestroy(graph);
+        if (node && st == cudaSuccess) {
+            graph_device_src = graph;
+            stats_node = node;
+        } else {
+            cudaGraphDestroy(graph);
+        }
         if (st != cudaSuccess) {
             cudaGetLastError();
             return false;
@@ -259,10 +318,9 @@ Plan* Plan::create(const std::vector<PlanFrame>& frames, const PlanConfig& confi
     const size_t states_at = carve.take(im.states_bytes + im.queue_bytes);
     im.result_stride = align_up(result_bytes(md), 256);
     im.results_bytes = im.result_stride * nf;
-    const size_t results_at = carve.take(im.results_bytes);
     const size_t desc_at = carve.take(sizeof(BatchDesc));
     const size_t io_fixed_at = carve.take(sizeof(FrameIO) * nf);
-    const size_t io_caller_at = carve.take(sizeof(FrameIO) * nf);
+    const size_t io_dev_at = carve.take(sizeof(FrameIO) * nf);
     int bands = 0;
     for (int i = 0; i < nf; ++i) {
         FrameDesc& d = hd.f[i];
@@ -323,10 +381,9 @@ Plan* Plan::create(const std::vector<PlanFrame>& frames, const PlanConfig& confi
     im.frames_dev = base + frames_at;
     im.states = reinterpret_cast<FrameState*>(base + states_at);
     im.queue = reinterpret_cast<WorkQueue*>(base + states_at + im.states_bytes);
-    im.results_dev = base + results_at;
     im.dev_desc = reinterpret_cast<BatchDesc*>(base + desc_at);
     im.io_fixed = reinterpret_cast<FrameIO*>(base + io_fixed_at);
-    im.io_caller = reinterpret_cast<FrameIO*>(base + io_caller_at);
+    im.io_dev = reinterpret_cast<FrameIO*>(base + io_dev_at);
     std::vector<FrameIO> fixed(nf);
     for (int i = 0; i < nf; ++i) {
         FrameDesc& d = hd.f[i];
@@ -351,14 +408,14 @@ Plan* Plan::create(const std::vector<PlanFrame>& frames, const PlanConfig& confi
         d.hull_quads = reinterpret_cast<float*>(base + off_hull[i]);
         d.quads = reinterpret_cast<float*>(base + off_quads[i]);
         d.decodes = reinterpret_cast<DecodeOut*>(base + off_dec[i]);
-        d.result = reinterpret_cast<FrameResultHeader*>(im.results_dev + im.result_stride * i);
         fixed[i].gray = im.frames_dev + im.frame_offset[i];
         fixed[i].stride = frames[i].width;
+        im.io_fixed_args.f[i] = fixed[i];
     }
     st = cudaHostAlloc(reinterpret_cast<void**>(&im.frames_pinned), frame_total, cudaHostAllocPortable);
     if (st == cudaSuccess)
         st = cudaHostAlloc(reinterpret_cast<void**>(&im.results_pinned), im.results_bytes,
-                           cudaHostAllocPortable);
+                           cudaHostAllocPortable | cudaHostAllocMapped);
     if (st == cudaSuccess)
         st = cudaHostAlloc(reinterpret_cast<void**>(&im.io_staging), sizeof(FrameIO) * nf,
                            cudaHostAllocPortable);
@@ -367,6 +424,16 @@ Plan* Plan::create(const std::vector<PlanFrame>& frames, const PlanConfig& confi
         return fail(cuda_error("cudaHostAlloc", st));
     }
     std::memset(im.results_pinned, 0, im.results_bytes);
+    void* results_mapped = nullptr;
+    st = cudaHostGetDevicePointer(&results_mapped, im.results_pinned, 0);
+    if (st != cudaSuccess) {
+        cudaGetLastError();
+        return fail(cuda_error("cudaHostGetDevicePointer", st));
+    }
+    for (int i = 0; i < nf; ++i) {
+        hd.f[i].result = reinterpret_cast<FrameResultHeader*>(static_cast<uint8_t*>(results_mapped) +
+                                                              im.result_stride * i);
+    }
     st = cudaStreamCreateWithFlags(&im.stream, cudaStreamNonBlocking);
     if (st == cudaSuccess) st = cudaStreamCreateWithFlags(&im.branch, cudaStreamNonBlocking);
     if (st == cudaSuccess) st = cudaEventCreateWithFlags(&im.ev_fork, cudaEventDisableTiming);
@@ -378,7 +445,6 @@ Plan* Plan::create(const std::vector<PlanFrame>& frames, const PlanConfig& confi
     if (st == cudaSuccess)
         st = cudaMemcpy(im.io_fixed, fixed.data(), sizeof(FrameIO) * nf, cudaMemcpyHostToDevice);
     if (st == cudaSuccess) st = cudaMemset(im.frames_dev, 0, frame_total);
-    if (st == cudaSuccess) st = cudaMemset(im.results_dev, 0, im.results_bytes);
     if (st != cudaSuccess) return fail(cuda_error("cudaMemcpy(plan)", st));
     for (int i = 0; i < nf; ++i) {
         im.io_staging[i].gray = fixed[i].gray;

@@ -42,8 +42,10 @@ const char* const kStageNames[kStageCount] = {
     "stats", "binarize_runs", "merge", "region_stats", "cand_count",
     "fit_decode_big", "fit_decode", "finalize"};
 
-void enqueue_pipeline(const BatchDesc* dd, const BatchDesc& hd, const FrameIO* io, void* stream_ptr,
-                      const LaunchConfig& lc, int sm_count, const ForkJoin* fork,
+const void* stats_kernel() { return reinterpret_cast<const void*>(k_stats); }
+
+void enqueue_pipeline(const BatchDesc* dd, const BatchDesc& hd, const FrameIOArgs& frames, FrameIO* io,
+                      void* stream_ptr, const LaunchConfig& lc, int sm_count, const ForkJoin* fork,
                       void* const* stage_events) {
     cudaStream_t s = static_cast<cudaStream_t>(stream_ptr);
     auto mark = [&](int k) {
@@ -58,7 +60,7 @@ void enqueue_pipeline(const BatchDesc* dd, const BatchDesc& hd, const FrameIO* i
     const int quad_grid =
         std::max(1, std::min((items + warps - 1) / warps, sm_count * lc.quad_ctas_per_sm));
     mark(0);
-    k_stats<<<hd.stats_ctas, 256, 0, s>>>(dd, io);
+    k_stats<<<hd.stats_ctas, 256, 0, s>>>(dd, frames, io);
     mark(1);
     int words_max = 1;
     for (int f = 0; f < hd.frames; ++f) words_max = std::max(words_max, hd.f[f].words);

@@ -7,7 +7,8 @@
 namespace bdgb {
 
 __global__ void __launch_bounds__(256) k_stats(const BatchDesc* __restrict__ b,
-                                               const FrameIO* __restrict__ io) {
+                                               const __grid_constant__ FrameIOArgs io,
+                                               FrameIO* __restrict__ io_out) {
     __shared__ StatsSmem sm;
     int fi = 0;
     {
@@ -18,8 +19,10 @@ __global__ void __launch_bounds__(256) k_stats(const BatchDesc* __restrict__ b,
         }
         fi = lo;
     }
-    if (!io[fi].gray) return;  // slot not used in this launch
-    stage_stats(b, io, fi, blockIdx.x - b->stats_prefix[fi], sm);
+    if (blockIdx.x == 0 && static_cast<int>(threadIdx.x) < b->frames) io_out[threadIdx.x] = io.f[threadIdx.x];
+    const FrameIO frame = io.f[fi];
+    if (!frame.gray) return;  // slot not used in this launch
+    stage_stats(b, frame, fi, blockIdx.x - b->stats_prefix[fi], sm);
 }
 
 __global__ void __launch_bounds__(256, 6) k_binarize_runs(const BatchDesc* __restrict__ b,

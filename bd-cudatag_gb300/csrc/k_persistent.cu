@@ -80,8 +80,8 @@ __device__ __forceinline__ uint32_t seed_item(const BatchDesc* b, uint32_t pos) 
 // Gives up the launch: the status says why, every frame's header carries it
 // (FrameResultHeader::pad), and every CTA leaves at its next claim.
 __device__ void abandon(const BatchDesc* b, WorkQueue* q, uint32_t why) {
-    atomicOr(&q->status, why);
-    for (int f = 0; f < b->frames; ++f) atomicOr(&b->f[f].result->pad, why);
+    const uint32_t all = atomicOr(&q->status, why) | why;
+    for (int f = 0; f < b->frames; ++f) *reinterpret_cast<volatile uint32_t*>(&b->f[f].result->pad) = all;
     __threadfence();
     atomicExch(&q->finished, 1u);
 }
@@ -211,7 +211,7 @@ k_persistent(const BatchDesc* __restrict__ b, const FrameIO* __restrict__ io, Wo
             case kStats: {
                 const uint32_t units = static_cast<uint32_t>(b->stats_prefix[fi + 1] - b->stats_prefix[fi]);
                 const bool used = io[fi].gray != nullptr;
-                if (used) stage_stats(b, io, fi, static_cast<int>(idx), *reinterpret_cast<StatsSmem*>(dyn));
+                if (used) stage_stats(b, io[fi], fi, static_cast<int>(idx), *reinterpret_cast<StatsSmem*>(dyn));
                 if (finish_unit(&st->done_stats, units, &ps.flag)) {
                     if (used) {
                         publish(b, q, kBin, fi, th, pp.stall_frame == fi, &ps.base);

@@ -43,7 +43,7 @@ __host__ __device__ constexpr size_t band_smem_bytes(int cap, int words) {
 
 constexpr int kFinalThreads = 256;
 
-__global__ void k_stats(const BatchDesc* b, const FrameIO* io);
+__global__ void k_stats(const BatchDesc* b, const __grid_constant__ FrameIOArgs io, FrameIO* io_out);
 __global__ void k_binarize_runs(const BatchDesc* b, const FrameIO* io, int cap, int bits_words);
 __global__ void k_merge(const BatchDesc* b, const FrameIO* io, int row_cap_max);
 __global__ void k_region_stats(const BatchDesc* b, const FrameIO* io);

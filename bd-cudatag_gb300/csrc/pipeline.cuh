@@ -104,6 +104,11 @@ struct FrameIO {
     int64_t stride;
 };
 
+// The same for every frame of a call, as a kernel argument.
+struct FrameIOArgs {
+    FrameIO f[kMaxFrames];
+};
+
 struct FrameDesc {
     int32_t width, height;
     int32_t tile_w, tile_h, words, row_cap;
@@ -138,7 +143,7 @@ struct FrameDesc {
     float* hull_quads;             // max_candidates * 8
     float* quads;                  // 2 * max_candidates * 8 (per family)
     DecodeOut* decodes;            // 2 * max_candidates
-    FrameResultHeader* result;     // header + 2 * max_detections records
+    FrameResultHeader* result;     // header + 2 * max_detections records (page-locked host memory)
 };
 
 struct BatchDesc {
@@ -193,8 +198,10 @@ BDGB_HD inline size_t result_bytes(int max_detections) {
     return sizeof(FrameResultHeader) + 2 * static_cast<size_t>(max_detections) * sizeof(bd_detection);
 }
 
-// Launch sequence of one batch on one stream (k_finalize.cu).  `io` is a
-// device array of FrameIO, one per frame.  With `fork` the big-candidate
+// Launch sequence of one batch on one stream (k_finalize.cu).  The frames'
+// pointers are an argument of the first kernel, which also writes them to
+// `device_io` for the others: a copy of 64 bytes to the device ahead of it
+// took 3.5 us of every batch (graph of eight empty kernels: 9.4 us, with the copy 12.9).  With `fork` the big-candidate
 // kernel runs on fork->stream beside the warp-per-candidate kernel.  When
 // stage_events is not null (no fork then) it holds kStageCount + 1
 // cudaEvent_t, recorded before the first kernel and after every kernel, so
@@ -210,9 +217,11 @@ struct PersistParams {
 // Per-device kernel attributes; call with the device current before the
 // first enqueue.  0 on success.
 int prepare_pipeline();
+// The first kernel of the sequence, to find its node in a captured graph.
+const void* stats_kernel();
 extern const char* const kStageNames[kStageCount];
 void enqueue_pipeline(const BatchDesc* device_desc, const BatchDesc& host_desc,
-                      const FrameIO* device_io, void* stream, const LaunchConfig& launch,
+                      const FrameIOArgs& io, FrameIO* device_io, void* stream, const LaunchConfig& launch,
                       int sm_count, const ForkJoin* fork, void* const* stage_events = nullptr);
 
 // The persistent launch of a batch (k_persistent.cu): one kernel whose CTAs

@@ -59,8 +59,8 @@ struct CandSmem {
 //    `stats_rows` tile rows; thread i of the CTA takes tile pair i (two
 //    horizontally adjacent tiles, 128-bit loads), row-major over those rows.
 // ===========================================================================
-__device__ __forceinline__ void stage_stats(const BatchDesc* __restrict__ b, const FrameIO* __restrict__ io, int fi,
-                            int cta, StatsSmem& sm) {
+__device__ __forceinline__ void stage_stats(const BatchDesc* __restrict__ b, const FrameIO& io, int fi, int cta,
+                            StatsSmem& sm) {
     uint32_t* s_span = sm.span;
     uint32_t* s_mean = sm.mean;
     int* s_lo = sm.lo;
@@ -79,8 +79,8 @@ __device__ __forceinline__ void stage_stats(const BatchDesc* __restrict__ b, con
     }
     __syncthreads();
 
-    const uint8_t* gray = io[fi].gray;
-    const int64_t stride = io[fi].stride;
+    const uint8_t* gray = io.gray;
+    const int64_t stride = io.stride;
     const int W = d.width, H = d.height, tw = d.tile_w;
     const bool vec16 = ((reinterpret_cast<uintptr_t>(gray) | static_cast<uintptr_t>(stride)) & 15u) == 0;
     const int pairs = (tw + 1) >> 1;

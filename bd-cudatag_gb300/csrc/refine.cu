@@ -11,14 +11,16 @@
 // with I the frame sampled bilinearly by the reference's formula and out-of-
 // frame samples masked (r_s = 0).  Loss = 0.5 * sum r_s^2 per quad.
 //
-// Derivatives: d(x, y)/dc comes from forward-mode duals through the closed
-// form (8 derivative lanes); dI/d(x, y) is the bilinear patch gradient.  The
+// Derivatives: dH/dc comes from forward-mode duals through the closed form,
+// one corner coordinate per lane; dI/d(x, y) is the bilinear patch gradient.  The
 // adjoint kernel returns dL/dc and scatters dL/dI onto the four pixels of
-// every sample.  The Gauss-Newton kernel builds J^T J and J^T r per quad,
-// solves the damped 8x8 system in FP64 and iterates in shared memory.
+// every sample.  The Gauss-Newton kernel sums its normal equations over the
+// homography's parameters, carries them over to the corners and solves the damped
+// 8x8 system in FP64, and iterates in shared memory.
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 
 #include "bdcudatag/bdcudatag.h"
@@ -33,76 +35,47 @@ namespace {
 
 constexpr int kThreads = 256;
 
+// A value and its derivative with respect to one corner coordinate.
 struct Dual {
-    float v;
-    float d[8];
+    float v, d;
 };
 
-__device__ __forceinline__ Dual dconst(float v) {
-    Dual r;
-    r.v = v;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) r.d[k] = 0.0f;
-    return r;
-}
+__device__ __forceinline__ Dual operator+(const Dual& a, const Dual& b) { return {a.v + b.v, a.d + b.d}; }
 
-__device__ __forceinline__ Dual dvar(float v, int k) {
-    Dual r = dconst(v);
-    r.d[k] = 1.0f;
-    return r;
-}
-
-__device__ __forceinline__ Dual operator+(const Dual& a, const Dual& b) {
-    Dual r;
-    r.v = a.v + b.v;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) r.d[k] = a.d[k] + b.d[k];
-    return r;
-}
-
-__device__ __forceinline__ Dual operator-(const Dual& a, const Dual& b) {
-    Dual r;
-    r.v = a.v - b.v;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) r.d[k] = a.d[k] - b.d[k];
-    return r;
-}
+__device__ __forceinline__ Dual operator-(const Dual& a, const Dual& b) { return {a.v - b.v, a.d - b.d}; }
 
 __device__ __forceinline__ Dual operator*(const Dual& a, const Dual& b) {
-    Dual r;
-    r.v = a.v * b.v;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) r.d[k] = a.d[k] * b.v + a.v * b.d[k];
-    return r;
+    return {a.v * b.v, a.d * b.v + a.v * b.d};
 }
 
 __device__ __forceinline__ Dual operator/(const Dual& a, const Dual& b) {
-    Dual r;
-    r.v = a.v / b.v;
     const float inv2 = 1.0f / (b.v * b.v);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) r.d[k] = (a.d[k] * b.v - a.v * b.d[k]) * inv2;
-    return r;
+    return {a.v / b.v, (a.d * b.v - a.v * b.d) * inv2};
 }
 
-// H and dH/dc (8 x 8) of the reference closed form, h[8] = 1.
-__device__ bool homography_dual(const float* c, float h[8], float dh[8][8]) {
-    const Dual x0 = dvar(c[0], 0), y0 = dvar(c[1], 1);
-    const Dual x1 = dvar(c[2], 2), y1 = dvar(c[3], 3);
-    const Dual x2 = dvar(c[4], 4), y2 = dvar(c[5], 5);
-    const Dual x3 = dvar(c[6], 6), y3 = dvar(c[7], 7);
-    const Dual dx1 = x1 - x2, dx2 = x3 - x2, dx3 = x0 - x1 + x2 - x3;
-    const Dual dy1 = y1 - y2, dy2 = y3 - y2, dy3 = y0 - y1 + y2 - y3;
+// H of the reference closed form (h[8] = 1) and its derivatives with respect to
+// corner coordinate k.
+__device__ __forceinline__ bool homography_dual(const float* c, int k, Dual H[8]) {
+    Dual x[4], y[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        x[i] = {c[2 * i], k == 2 * i ? 1.0f : 0.0f};
+        y[i] = {c[2 * i + 1], k == 2 * i + 1 ? 1.0f : 0.0f};
+    }
+    const Dual dx1 = x[1] - x[2], dx2 = x[3] - x[2], dx3 = x[0] - x[1] + x[2] - x[3];
+    const Dual dy1 = y[1] - y[2], dy2 = y[3] - y[2], dy3 = y[0] - y[1] + y[2] - y[3];
     const Dual det = dx1 * dy2 - dx2 * dy1;
     if (fabsf(det.v) < 1e-9f) return false;
     const Dual g = (dx3 * dy2 - dx2 * dy3) / det;
-    const Dual k = (dx1 * dy3 - dx3 * dy1) / det;
-    const Dual H[8] = {x1 - x0 + g * x1, x3 - x0 + k * x3, x0, y1 - y0 + g * y1,
-                       y3 - y0 + k * y3, y0, g, k};
-    for (int i = 0; i < 8; ++i) {
-        h[i] = H[i].v;
-        for (int j = 0; j < 8; ++j) dh[i][j] = H[i].d[j];
-    }
+    const Dual h = (dx1 * dy3 - dx3 * dy1) / det;
+    H[0] = x[1] - x[0] + g * x[1];
+    H[1] = x[3] - x[0] + h * x[3];
+    H[2] = x[0];
+    H[3] = y[1] - y[0] + g * y[1];
+    H[4] = y[3] - y[0] + h * y[3];
+    H[5] = y[0];
+    H[6] = g;
+    H[7] = h;
     return true;
 }
 
@@ -191,7 +164,28 @@ __device__ void block_sum(float (&v)[N], float (*smem)[kThreads]) {
     __syncthreads();
 }
 
-__device__ bool load_quad(const bd_refine_args& a, int qi, const float* corners, QuadCtx* q) {
+// The quad's context into shared memory, by lanes 0-7 of the first warp (lane k
+// holds the derivatives with respect to corner coordinate k); *ok says whether
+// it has a homography.  The caller synchronises.
+__device__ __forceinline__ void load_quad(const bd_refine_args& a, int qi, const float* corners, QuadCtx* q,
+                                          int* ok) {
+    const int k = threadIdx.x;
+    if (k >= 8) return;
+    float c[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) c[i] = corners[i];
+    Dual H[8];
+    const bool good = homography_dual(c, k, H);
+    if (good) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) q->dh[i][k] = H[i].d;
+    }
+    if (k != 0) return;
+    *ok = good ? 1 : 0;
+    if (good) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) q->h[i] = H[i].v;
+    }
     q->image = a.images + static_cast<int64_t>(a.image_index ? a.image_index[qi] : 0) * a.image_pitch;
     q->width = a.width;
     q->height = a.height;
@@ -201,7 +195,6 @@ __device__ bool load_quad(const bd_refine_args& a, int qi, const float* corners,
     q->tmpl = a.templates + static_cast<int64_t>(qi) * a.cells * a.cells;
     q->lo = a.levels ? a.levels[2 * qi] : 0.0f;
     q->hi = a.levels ? a.levels[2 * qi + 1] : 255.0f;
-    return homography_dual(corners, q->h, q->dh);
 }
 
 __global__ void __launch_bounds__(kThreads) k_refine_forward(bd_refine_args a, float* residuals,
@@ -210,7 +203,7 @@ __global__ void __launch_bounds__(kThreads) k_refine_forward(bd_refine_args a, f
     __shared__ int ok;
     __shared__ float red[1][kThreads];
     const int qi = blockIdx.x;
-    if (threadIdx.x == 0) ok = load_quad(a, qi, a.corners + 8 * qi, &q) ? 1 : 0;
+    load_quad(a, qi, a.corners + 8 * qi, &q, &ok);
     __syncthreads();
     const int n = a.cells * a.cells * a.samples_per_cell * a.samples_per_cell;
     float acc[1] = {0.0f};
@@ -233,7 +226,7 @@ __global__ void __launch_bounds__(kThreads) k_refine_backward(bd_refine_args a,
     __shared__ int ok;
     __shared__ float red[8][kThreads];
     const int qi = blockIdx.x;
-    if (threadIdx.x == 0) ok = load_quad(a, qi, a.corners + 8 * qi, &q) ? 1 : 0;
+    load_quad(a, qi, a.corners + 8 * qi, &q, &ok);
     __syncthreads();
     const int n = a.cells * a.cells * a.samples_per_cell * a.samples_per_cell;
     float g[8] = {};
@@ -260,116 +253,398 @@ __global__ void __launch_bounds__(kThreads) k_refine_backward(bd_refine_args a,
     if (threadIdx.x < 8 && grad_corners) grad_corners[8 * qi + threadIdx.x] = g[threadIdx.x];
 }
 
-// Cholesky solve of (A + lambda * diag(A)) x = -b, 8 x 8, FP64.
-__device__ bool solve8(const double A[8][8], const double b[8], double lambda, double x[8]) {
-    double L[8][8] = {};
-    for (int i = 0; i < 8; ++i) {
-        for (int j = 0; j <= i; ++j) {
-            double s = A[i][j] + (i == j ? lambda * A[i][i] : 0.0);
-            for (int k = 0; k < j; ++k) s -= L[i][k] * L[j][k];
-            if (i == j) {
-                if (s <= 1e-12) return false;
-                L[i][i] = sqrt(s);
-            } else {
-                L[i][j] = s / L[j][j];
-            }
+// ---------------------------------------------------------------------------
+// Gauss-Newton.
+//
+// With w = dr/dH of a sample (8 numbers), its row of J is dH^T w, dH = dH/dc
+// (8 x 8, the same for every sample).  So the samples sum w w^T and w r, and the
+// sums are carried over to the corners once per iteration, instead of every
+// sample forming its row of J.  w is made of three numbers -- A = I_x / den, B =
+// I_y / den, C = -(A x + B y) -- times u, v and 1, and a thread keeps to one
+// column of the sample grid (one u), so a sample adds six products times 1, v and
+// v^2, and u enters when the column is done.
+//
+// The photometric levels (mean intensity over the black and the white cells) are
+// not known before the samples are read.  The sums are taken against provisional levels (the last
+// iteration's; at first 0 and 255) and corrected by what the true ones differ from
+// them: one pass over the samples where there were two.
+//
+// Sample positions are relative to a whole pixel near the quad's centre: near
+// 1000 px they would carry 6e-5 px of rounding, and the parts of J^T J would
+// cancel.
+//
+// Bound: issue slots and L1 passes of the samples (some 100 instructions, 355
+// before), then the serial chain between two iterations (reduction, transform, FP64 solve: 40%).
+// 256 quads of 80 x 80 samples, 5 iterations: 792 us before, 120 us (170 us with 32
+// columns of one row to a warp).  Corners are five times nearer to 64-bit arithmetic.
+// ---------------------------------------------------------------------------
+constexpr int kMaxGrid = 256;     // samples per side: 16 cells of 16
+constexpr int kSums = 64;         // 61 used
+// A warp takes 8 columns by 4 rows of samples at a time: neighbouring pixels, so
+// a load meets some 8 rows of the frame.  32 columns of one sample row meet up to 28
+// when the quad lies askew, and L1 takes a pass per row.
+constexpr int kTileCols = 8, kTileRows = 4;
+constexpr int kGnWarps = 10;      // 10 x 8 columns: 10 cells of 8 samples (tag36h11)
+
+// Places of the sums.  Products: the unique entries of w w^T by pair and powers
+// of (u, v); then w r, w over white samples, w over all, then per colour (black,
+// white) the count and the first two moments of value - provisional level.
+enum SumAt {
+    kAA = 0, kBB = 6, kAB = 12,  // uu, uv, u, vv, v, 1
+    kAC = 18, kBC = 23,          // uu, uv, u, vv, v
+    kCC = 28,                    // uu, uv, vv
+    kWR = 31, kWW = 39, kWAll = 47,
+    kCount = 55, kMoment1 = 57, kMoment2 = 59
+};
+
+// Sum over the lanes of a warp of each of 64 values: 63 shuffles (value pairs are
+// split between the halves of the warp, then the quarters ...) where a
+// tree per value takes 320.  Lane l is left with the sums of values l and l + 32 in
+// v[0] and v[1].
+__device__ __forceinline__ void warp_sums(float (&v)[kSums], int lane) {
+#pragma unroll
+    for (int off = 1, n = kSums / 2; off < 32; off <<= 1, n >>= 1) {
+        const bool up = (lane & off) != 0;
+#pragma unroll
+        for (int i = 0; i < n; ++i) {
+            const float keep = up ? v[2 * i + 1] : v[2 * i];
+            const float send = up ? v[2 * i] : v[2 * i + 1];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
         }
     }
-    double y[8];
-    for (int i = 0; i < 8; ++i) {
-        double s = -b[i];
-        for (int k = 0; k < i; ++k) s -= L[i][k] * y[k];
-        y[i] = s / L[i][i];
+}
+
+struct GnSmem {
+    float h[8];
+    float dh[8][8];               // dH_i / dc_k
+    float c[8];                   // corners
+    float level[2];               // provisional: black, white
+    int cx, cy;
+    int ok;
+    float v[kMaxGrid];            // v of each sample row
+    uint16_t cell_bit[kMaxGrid];  // 1 << its cell
+    uint32_t white[16];           // bit cy of white[cx]: a white cell
+    float part[kGnWarps][kSums];
+    float sum[kSums];
+    double shift[2];              // true levels - provisional ones
+    float t[8][8];                // W dH
+    double wr[8];                 // sum of w r against the true levels
+    double l[8][8];               // the solve's factor
+};
+
+// Place in the sums of w_i w_j (parameters in order: A u, A v, A, B u, B v, B, C u, C v).
+__device__ __forceinline__ int product_at(int i, int j) {
+    if (i > j) {
+        const int t = i;
+        i = j;
+        j = t;
     }
-    for (int i = 7; i >= 0; --i) {
-        double s = y[i];
-        for (int k = i + 1; k < 8; ++k) s -= L[k][i] * x[k];
-        x[i] = s / L[i][i];
+    const int pi = i / 3, pj = j / 3;          // A, B, C
+    const int mi = i - 3 * pi, mj = j - 3 * pj;  // u, v, 1
+    const int lo = min(mi, mj), hi = max(mi, mj);
+    // uu, uv, u, vv, v, 1 by (lo, hi) = (0,0) (0,1) (0,2) (1,1) (1,2) (2,2)
+    const int m = lo == 0 ? hi : lo + hi + 1;
+    if (pi == 0) return (pj == 0 ? kAA : (pj == 1 ? kAB : kAC)) + m;
+    if (pi == 1) return (pj == 1 ? kBB : kBC) + m;
+    return kCC + (m == 3 ? 2 : m);
+}
+
+__device__ __forceinline__ double shfl_double(double v, int lane) { return __shfl_sync(0xffffffffu, v, lane); }
+
+// 1 / d for d > 0 in float's range: Newton steps from the float reciprocal (24
+// good bits, then 48, then all).  FP64 is narrow on this GPU: a division is
+// twice as many of its instructions.
+__device__ __forceinline__ double reciprocal(double d) {
+    double r = static_cast<double>(__frcp_rn(static_cast<float>(d)));
+    r = __fma_rn(r, __fma_rn(-d, r, 1.0), r);
+    return __fma_rn(r, __fma_rn(-d, r, 1.0), r);
+}
+
+// One warp: (M + lambda diag(M)) x = -b by LDL^T in FP64, lane i = row i (lanes 8
+// and up repeat lanes 0-7).  False when a pivot is not positive.
+__device__ __forceinline__ bool solve8(double (&row)[8], double b, double lambda, int lane, double (*l_out)[8],
+                                       double* x) {
+    const int i = lane & 7;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        if (i == j) row[j] = __fma_rn(lambda, row[j], row[j]);
     }
+    double y = -b;
+    double inv_own = 0.0;
+    bool good = true;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const double pivot = shfl_double(row[j], j);
+        good = good && pivot > 1e-12;
+        const double inv = reciprocal(pivot);
+        if (i == j) inv_own = inv;
+        const double l = row[j] * inv;
+        const double yj = shfl_double(y, j);
+        if (i > j) y = __fma_rn(-l, yj, y);
+#pragma unroll
+        for (int k = j + 1; k < 8; ++k) {
+            const double skj = shfl_double(row[j], k);  // row k, column j
+            if (i > j) row[k] = __fma_rn(-l, skj, row[k]);
+        }
+        if (lane < 8) l_out[lane][j] = l;
+    }
+    __syncwarp();
+    if (!good) return false;
+    double z = y * inv_own;
+    // x_i = z_i - sum over k > i of L[k][i] x_k, from the last row up.
+#pragma unroll
+    for (int k = 7; k > 0; --k) {
+        const double xk = shfl_double(z, k);
+        if (i < k) z = __fma_rn(-l_out[k][i], xk, z);
+    }
+    *x = z;
     return true;
 }
 
-__global__ void __launch_bounds__(kThreads) k_refine_gauss_newton(bd_refine_args a, float* corners,
-                                                                  int iterations, float* loss) {
-    __shared__ QuadCtx q;
-    __shared__ float c[8];
-    __shared__ int ok;
-    __shared__ float red[44][kThreads];
+__global__ void __launch_bounds__(kGnWarps * 32, 2) k_refine_gauss_newton(bd_refine_args a, float* corners,
+                                                                     int iterations, float* loss) {
+    __shared__ GnSmem sm;
     const int qi = blockIdx.x;
-    const int n = a.cells * a.cells * a.samples_per_cell * a.samples_per_cell;
-    if (threadIdx.x < 8) c[threadIdx.x] = corners[8 * qi + threadIdx.x];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int warps = blockDim.x >> 5;
+    const int grid = a.cells * a.samples_per_cell;
+    const float dim = static_cast<float>(a.cells - 2);
+    const uint8_t* image = a.images + static_cast<int64_t>(a.image_index ? a.image_index[qi] : 0) * a.image_pitch;
+    const uint8_t* tmpl = a.templates + static_cast<int64_t>(qi) * a.cells * a.cells;
+
+    // Sample coordinate i of the grid's side (cell, sub-sample).
+    auto coordinate = [&](int i) {
+        const int cell = i / a.samples_per_cell;
+        const int sub = i - cell * a.samples_per_cell;
+        return (static_cast<float>(cell - 1) + (static_cast<float>(sub) + 0.5f) / a.samples_per_cell) / dim;
+    };
+    for (int i = tid; i < grid; i += blockDim.x) {
+        sm.v[i] = coordinate(i);
+        sm.cell_bit[i] = static_cast<uint16_t>(1u << (i / a.samples_per_cell));
+    }
+    if (tid < 16) sm.white[tid] = 0;
+    if (tid == 0) {
+        const float* c = corners + 8 * qi;
+        sm.cx = static_cast<int>(floorf(0.25f * (c[0] + c[2] + c[4] + c[6])));
+        sm.cy = static_cast<int>(floorf(0.25f * (c[1] + c[3] + c[5] + c[7])));
+        sm.level[0] = a.levels ? a.levels[2 * qi] : 0.0f;
+        sm.level[1] = a.levels ? a.levels[2 * qi + 1] : 255.0f;
+    }
     __syncthreads();
-    float last_loss = 0.0f;
+    if (tid < 8) sm.c[tid] = corners[8 * qi + tid];
+    for (int i = tid; i < a.cells * a.cells; i += blockDim.x) {
+        const int cy = i / a.cells;
+        if (tmpl[i]) atomicOr(&sm.white[i - cy * a.cells], 1u << cy);
+    }
+    __syncthreads();
+    // The columns in blocks of 8, `share` warps to a block (each takes its part of
+    // the rows), or several blocks to a warp one after another.
+    const int blocks = (grid + kTileCols - 1) / kTileCols;
+    const int share = max(1, warps / blocks);
+    const int row0 = (warp % share) * kTileRows + (lane >> 3);
+    const int row_step = share * kTileRows;
+    const int ox = sm.cx, oy = sm.cy;
+    const unsigned in_x = static_cast<unsigned>(a.width - 1), in_y = static_cast<unsigned>(a.height - 1);
+
+    bool measured = false;  // the sums are those of a homography's samples
     for (int it = 0; it <= iterations; ++it) {
-        if (threadIdx.x == 0) ok = load_quad(a, qi, c, &q) ? 1 : 0;
-        __syncthreads();
-        if (!ok) break;
-        // Photometric levels: mean intensity over black / white template cells.
-        float lv[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        if (!a.levels) {
-            for (int s = threadIdx.x; s < n; s += kThreads) {
-                Sample smp;
-                eval_sample(q, s, false, &smp);
-                if (!smp.in) continue;
-                const int cell = s / (a.samples_per_cell * a.samples_per_cell);
-                lv[q.tmpl[cell] ? 2 : 0] += smp.val;
-                lv[q.tmpl[cell] ? 3 : 1] += 1.0f;
-            }
-            block_sum<4>(lv, reinterpret_cast<float(*)[kThreads]>(red));
-            if (threadIdx.x == 0) {
-                q.lo = lv[1] > 0.0f ? lv[0] / lv[1] : 0.0f;
-                q.hi = lv[3] > 0.0f ? lv[2] / lv[3] : 255.0f;
-            }
-            __syncthreads();
-        }
-        // Normal equations: 36 unique entries of J^T J, 8 of J^T r, loss.
-        float acc[45] = {};
-        for (int s = threadIdx.x; s < n; s += kThreads) {
-            Sample smp;
-            eval_sample(q, s, true, &smp);
-            if (!smp.in) continue;
-            int m = 0;
+        if (tid < 8) {
+            float c[8];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
+            for (int i = 0; i < 8; ++i) c[i] = sm.c[i] - static_cast<float>((i & 1) ? oy : ox);
+            Dual H[8];
+            const bool good = homography_dual(c, tid, H);
+            if (tid == 0) sm.ok = good ? 1 : 0;
+            if (good) {
 #pragma unroll
-                for (int j = 0; j <= i; ++j) acc[m++] += smp.gx[i] * smp.gx[j];
-            }
-#pragma unroll
-            for (int i = 0; i < 8; ++i) acc[36 + i] += smp.gx[i] * smp.r;
-            acc[44] += 0.5f * smp.r * smp.r;
-        }
-        float part1[22], part2[23];
-#pragma unroll
-        for (int i = 0; i < 22; ++i) part1[i] = acc[i];
-#pragma unroll
-        for (int i = 0; i < 23; ++i) part2[i] = acc[22 + i];
-        block_sum<22>(part1, red);
-        block_sum<23>(part2, red);
-        last_loss = part2[22];
-        if (it == iterations) break;
-        if (threadIdx.x == 0) {
-            double A[8][8], b[8], x[8];
-            int m = 0;
-            for (int i = 0; i < 8; ++i) {
-                for (int j = 0; j <= i; ++j) {
-                    const float v = m < 22 ? part1[m] : part2[m - 22];
-                    A[i][j] = A[j][i] = v;
-                    ++m;
-                }
-            }
-            for (int i = 0; i < 8; ++i) b[i] = part2[14 + i];
-            if (solve8(A, b, 1e-4, x)) {
                 for (int i = 0; i < 8; ++i) {
-                    // Steps are clamped to 2 px per coordinate.
-                    const double step = fmin(fmax(x[i], -2.0), 2.0);
-                    c[i] = static_cast<float>(c[i] + step);
+                    sm.dh[i][tid] = H[i].d;
+                    if (tid == 0) sm.h[i] = H[i].v;
                 }
             }
         }
+        __syncthreads();
+        if (!sm.ok) break;
+        const float h1 = sm.h[1], h4 = sm.h[4], h7 = sm.h[7];
+        const float level_b = sm.level[0], level_w = sm.level[1];
+        for (int block = warp / share; block < blocks; block += warps) {
+            const int col = block * kTileCols + (lane & 7);
+            const float u = sm.v[min(col, grid - 1)];  // the grid is square: u and v share their values
+            const uint32_t white_cells = sm.white[min(col, grid - 1) / a.samples_per_cell];
+            const float hx = __fmaf_rn(sm.h[0], u, sm.h[2]);
+            const float hy = __fmaf_rn(sm.h[3], u, sm.h[5]);
+            const float hd = __fmaf_rn(sm.h[6], u, 1.0f);
+            float p0[6] = {}, p1[6] = {}, p2[6] = {};      // AA, BB, AB, AC, BC, CC by powers of v
+            float r0[3] = {}, r1[3] = {};                  // (A, B, C) r
+            float w0[3] = {}, w1[3] = {};                  // (A, B, C), white samples
+            float s0[3] = {}, s1[3] = {};                  // (A, B, C), all
+            float count[2] = {}, m1[2] = {}, m2[2] = {};
+            for (int j = col < grid ? row0 : grid; j < grid; j += row_step) {
+                const float v = sm.v[j];
+                const float den = __fmaf_rn(h7, v, hd);
+                const float inv = __frcp_rn(den);
+                const float x = __fmaf_rn(h1, v, hx) * inv;
+                const float y = __fmaf_rn(h4, v, hy) * inv;
+                const float fx0 = floorf(x), fy0 = floorf(y);
+                const int ix = static_cast<int>(fx0) + ox, iy = static_cast<int>(fy0) + oy;
+                if (!(den > 1e-6f) || static_cast<unsigned>(ix) >= in_x || static_cast<unsigned>(iy) >= in_y) continue;
+                const float fx = x - fx0, fy = y - fy0;
+                const uint8_t* p = image + (static_cast<int64_t>(iy) * a.stride + ix);
+                const float pa = __ldg(p), pb = __ldg(p + 1);
+                const float pc = __ldg(p + a.stride), pd = __ldg(p + a.stride + 1);
+                const float top = __fmaf_rn(pb - pa, fx, pa);
+                const float bottom = __fmaf_rn(pd - pc, fx, pc);
+                const float value = __fmaf_rn(bottom - top, fy, top);
+                const float A = __fmaf_rn((pd - pc) - (pb - pa), fy, pb - pa) * inv;
+                const float B = (bottom - top) * inv;
+                const float C = -__fmaf_rn(A, x, B * y);
+                const bool white = (white_cells & sm.cell_bit[j]) != 0;
+                const float r = value - (white ? level_w : level_b);
+                const float vv = v * v;
+                const float pr[6] = {A * A, B * B, A * B, A * C, B * C, C * C};
+#pragma unroll
+                for (int i = 0; i < 6; ++i) {
+                    p0[i] += pr[i];
+                    p1[i] = __fmaf_rn(pr[i], v, p1[i]);
+                    p2[i] = __fmaf_rn(pr[i], vv, p2[i]);
+                }
+                const float abc[3] = {A, B, C};
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    const float ar = abc[i] * r;
+                    r0[i] += ar;
+                    r1[i] = __fmaf_rn(ar, v, r1[i]);
+                    s0[i] += abc[i];
+                    s1[i] = __fmaf_rn(abc[i], v, s1[i]);
+                    const float aw = white ? abc[i] : 0.0f;
+                    w0[i] += aw;
+                    w1[i] = __fmaf_rn(aw, v, w1[i]);
+                }
+                const float rw = white ? r : 0.0f, rb = white ? 0.0f : r;
+                count[0] += white ? 0.0f : 1.0f;
+                count[1] += white ? 1.0f : 0.0f;
+                m1[0] += rb;
+                m1[1] += rw;
+                m2[0] = __fmaf_rn(rb, rb, m2[0]);
+                m2[1] = __fmaf_rn(rw, rw, m2[1]);
+            }
+            // The column's u, then the sums over the CTA.
+            float sums[kSums] = {};
+            const float uu = u * u;
+            const int pair_at[3] = {kAA, kBB, kAB};
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                sums[pair_at[i] + 0] = uu * p0[i];
+                sums[pair_at[i] + 1] = u * p1[i];
+                sums[pair_at[i] + 2] = u * p0[i];
+                sums[pair_at[i] + 3] = p2[i];
+                sums[pair_at[i] + 4] = p1[i];
+                sums[pair_at[i] + 5] = p0[i];
+            }
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const int at = i == 0 ? kAC : kBC;
+                sums[at + 0] = uu * p0[3 + i];
+                sums[at + 1] = u * p1[3 + i];
+                sums[at + 2] = u * p0[3 + i];
+                sums[at + 3] = p2[3 + i];
+                sums[at + 4] = p1[3 + i];
+            }
+            sums[kCC + 0] = uu * p0[5];
+            sums[kCC + 1] = u * p1[5];
+            sums[kCC + 2] = p2[5];
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                sums[kWR + 3 * i] = u * r0[i];
+                sums[kWR + 3 * i + 1] = r1[i];
+                sums[kWW + 3 * i] = u * w0[i];
+                sums[kWW + 3 * i + 1] = w1[i];
+                sums[kWAll + 3 * i] = u * s0[i];
+                sums[kWAll + 3 * i + 1] = s1[i];
+                if (i < 2) {
+                    sums[kWR + 3 * i + 2] = r0[i];
+                    sums[kWW + 3 * i + 2] = w0[i];
+                    sums[kWAll + 3 * i + 2] = s0[i];
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                sums[kCount + i] = count[i];
+                sums[kMoment1 + i] = m1[i];
+                sums[kMoment2 + i] = m2[i];
+            }
+            warp_sums(sums, lane);
+            const bool first = block == warp / share;
+            sm.part[warp][lane] = first ? sums[0] : sm.part[warp][lane] + sums[0];
+            sm.part[warp][lane + 32] = first ? sums[1] : sm.part[warp][lane + 32] + sums[1];
+        }
+        __syncthreads();
+        if (tid < kSums) {
+            float t = 0.0f;
+            for (int k = 0; k < warps; ++k) t += sm.part[k][tid];
+            sm.sum[tid] = t;
+        }
+        __syncthreads();
+        // T = W dH (entry (i, k) by thread 8 i + k); the true levels, as shifts
+        // of the provisional ones, by two threads of another warp.
+        if (tid < 64) {
+            const int i = tid >> 3, k = tid & 7;
+            float t = 0.0f;
+#pragma unroll
+            for (int m = 0; m < 8; ++m) t = __fmaf_rn(sm.sum[product_at(i, m)], sm.dh[m][k], t);
+            sm.t[i][k] = t;
+        } else if (tid < 66) {
+            const int i = tid - 64;
+            const bool own = !a.levels && sm.sum[kCount + i] > 0.0f;
+            sm.shift[i] = own ? sm.sum[kMoment1 + i] * reciprocal(sm.sum[kCount + i]) : 0.0;
+        }
+        if (warp == 2) {
+            __syncwarp();
+            if (lane < 8) {
+                const double ww = sm.sum[kWW + lane];
+                sm.wr[lane] = sm.sum[kWR + lane] - sm.shift[1] * ww - sm.shift[0] * (sm.sum[kWAll + lane] - ww);
+            }
+        }
+        __syncthreads();
+        if (warp == 0) {
+            // Lane k (mod 8): row k of J^T J = dH^T T and of J^T r.
+            if (it < iterations) {
+                const int k = lane & 7;
+                float m[8] = {};
+                double b = 0.0;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const float d = sm.dh[i][k];
+                    b = __fma_rn(static_cast<double>(d), sm.wr[i], b);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) m[j] = __fmaf_rn(d, sm.t[i][j], m[j]);
+                }
+                double row[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) row[j] = static_cast<double>(m[j]);
+                double x = 0.0;
+                const bool solved = solve8(row, b, 1e-4, lane, sm.l, &x);
+                if (lane < 8 && solved) {
+                    // Steps are clamped to 2 px per coordinate.
+                    sm.c[lane] = static_cast<float>(sm.c[lane] + fmin(fmax(x, -2.0), 2.0));
+                }
+                if (lane < 2) sm.level[lane] = static_cast<float>(sm.level[lane] + sm.shift[lane]);
+            }
+        }
+        measured = true;
+        if (it == iterations) break;
         __syncthreads();
     }
-    if (threadIdx.x < 8) corners[8 * qi + threadIdx.x] = c[threadIdx.x];
-    if (threadIdx.x == 0 && loss) loss[qi] = last_loss;
+    if (tid < 8) corners[8 * qi + tid] = sm.c[tid];
+    if (tid == 0 && loss) {
+        // Half the sum of (r - shift)^2, at the last corners that had a homography.
+        double l = 0.0;
+        for (int i = 0; measured && i < 2; ++i) {
+            const double sh = sm.shift[i];
+            l += sm.sum[kMoment2 + i] - sh * (2.0 * sm.sum[kMoment1 + i] - sh * sm.sum[kCount + i]);
+        }
+        loss[qi] = static_cast<float>(0.5 * l);
+    }
 }
 
 int32_t check_args(const bd_refine_args* a) {
@@ -455,7 +730,11 @@ int32_t bd_refine_gauss_newton(const bd_refine_args* args, float* corners_inout,
         return BD_ERROR_INVALID_ARGUMENT;
     }
     if (args->count == 0) return BD_OK;
-    k_refine_gauss_newton<<<args->count, kThreads, 0, static_cast<cudaStream_t>(cuda_stream)>>>(
+    // A warp per block of columns, more when there are few blocks; at least the
+    // three warps that the steps between the samples use.
+    const int blocks = (args->cells * args->samples_per_cell + kTileCols - 1) / kTileCols;
+    const int warps = blocks >= kGnWarps ? kGnWarps : std::max(3, kGnWarps / blocks * blocks);
+    k_refine_gauss_newton<<<args->count, warps * 32, 0, static_cast<cudaStream_t>(cuda_stream)>>>(
         *args, corners_inout, iterations, loss);
     return launched();
 }

@@ -33,8 +33,6 @@ void set_last_error(const char* message);  // capi.cpp
 
 namespace {
 
-constexpr int kThreads = 256;
-
 // A value and its derivative with respect to one corner coordinate.
 struct Dual {
     float v, d;
@@ -79,178 +77,281 @@ __device__ __forceinline__ bool homography_dual(const float* c, int k, Dual H[8]
     return true;
 }
 
-struct Sample {
-    bool in;
-    float val;    // frame value at the sample
-    float r;      // residual
-    float gx[8];  // d r / d c
-    int64_t off;  // pixel offset of the top-left bilinear neighbour
-    float w[4];   // bilinear weights (a, b, c, d)
+// ---------------------------------------------------------------------------
+// The sample grid of a quad: `grid` x `grid` samples, grid = cells * samples per
+// cell.  A warp takes 8 columns by 4 rows at a time: neighbouring pixels, so a
+// load meets some 8 rows of the frame.  32 columns of one sample row meet up to 28
+// when the quad lies askew, and L1 takes a pass per row.  With 8 samples per cell
+// such a tile is also 32 consecutive samples of a residual array.  A thread keeps
+// to one column (one u) of a block of 8.
+// ---------------------------------------------------------------------------
+constexpr int kMaxGrid = 256;     // 16 cells of 16
+constexpr int kTileCols = 8, kTileRows = 4;
+
+// Warps for a grid of `side` samples, at most `most`: a multiple of its column
+// blocks, or `most` when there are more blocks than that.
+inline int grid_warps(int side, int most) {
+    const int blocks = (side + kTileCols - 1) / kTileCols;
+    return blocks >= most ? most : most / blocks * blocks;
+}
+
+// A thread's place: its warp takes column blocks block0, block0 + warps, ..., rows row0,
+// row0 + row_step, ...
+struct GridPlace {
+    int blocks, block0, row0, row_step;
 };
 
-struct QuadCtx {
-    const uint8_t* image;
-    int width, height;
-    int64_t stride;
-    float h[8];
-    float dh[8][8];
-    float lo, hi;
-    const uint8_t* tmpl;
-    int cells, spc;
+__device__ __forceinline__ GridPlace grid_place(int side) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+    GridPlace g;
+    g.blocks = (side + kTileCols - 1) / kTileCols;
+    const int share = max(1, warps / g.blocks);  // warps of one column block
+    g.block0 = warp / share;
+    g.row0 = (warp % share) * kTileRows + (lane >> 3);
+    g.row_step = share * kTileRows;
+    return g;
+}
+
+// Sample coordinate i of the grid's side (cell, sub-sample), in tag units.
+__device__ __forceinline__ float grid_coordinate(const bd_refine_args& a, int i) {
+    const int cell = i / a.samples_per_cell;
+    const int sub = i - cell * a.samples_per_cell;
+    return (static_cast<float>(cell - 1) + (static_cast<float>(sub) + 0.5f) / a.samples_per_cell) /
+           static_cast<float>(a.cells - 2);
+}
+
+struct GridSmem {
+    float v[kMaxGrid];            // coordinate of each sample row (and column)
+    uint16_t cell_bit[kMaxGrid];  // 1 << its cell
+    uint32_t white[16];           // bit cy of white[cx]: a white cell
 };
 
-// Sample s of the quad: position through H, bilinear value, gradient w.r.t.
-// the corners.
-__device__ __forceinline__ void eval_sample(const QuadCtx& q, int s, bool want_grad, Sample* out) {
-    const int per_cell = q.spc * q.spc;
-    const int cell = s / per_cell;
-    const int sub = s - cell * per_cell;
-    const int cy = cell / q.cells, cx = cell - cy * q.cells;
-    const int sy = sub / q.spc, sx = sub - sy * q.spc;
-    const float dim = static_cast<float>(q.cells - 2);
-    const float u = (static_cast<float>(cx - 1) + (static_cast<float>(sx) + 0.5f) / q.spc) / dim;
-    const float v = (static_cast<float>(cy - 1) + (static_cast<float>(sy) + 0.5f) / q.spc) / dim;
-    const float nx = q.h[0] * u + q.h[1] * v + q.h[2];
-    const float ny = q.h[3] * u + q.h[4] * v + q.h[5];
-    const float den = q.h[6] * u + q.h[7] * v + 1.0f;
-    const float x = nx / den, y = ny / den;
-    out->in = den > 1e-6f && x >= 0.0f && y >= 0.0f && x < static_cast<float>(q.width - 1) &&
-              y < static_cast<float>(q.height - 1);
-    out->r = 0.0f;
-    if (!out->in) return;
+// Fills the grid's tables (two barriers, the last one at the end).
+__device__ __forceinline__ void load_grid(const bd_refine_args& a, int qi, GridSmem& sm) {
+    const int tid = threadIdx.x;
+    const int side = a.cells * a.samples_per_cell;
+    for (int i = tid; i < side; i += blockDim.x) {
+        sm.v[i] = grid_coordinate(a, i);
+        sm.cell_bit[i] = static_cast<uint16_t>(1u << (i / a.samples_per_cell));
+    }
+    if (tid < 16) sm.white[tid] = 0;
+    __syncthreads();
+    const uint8_t* tmpl = a.templates + static_cast<int64_t>(qi) * a.cells * a.cells;
+    for (int i = tid; i < a.cells * a.cells; i += blockDim.x) {
+        const int cy = i / a.cells;
+        if (tmpl[i]) atomicOr(&sm.white[i - cy * a.cells], 1u << cy);
+    }
+    __syncthreads();
+}
+
+__device__ __forceinline__ const uint8_t* quad_image(const bd_refine_args& a, int qi) {
+    return a.images + static_cast<int64_t>(a.image_index ? a.image_index[qi] : 0) * a.image_pitch;
+}
+
+// Sum of one value per thread over the CTA (fixed order), in thread 0.
+__device__ __forceinline__ float cta_sum(float v, float* s_part) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+    if (lane == 0) s_part[warp] = v;
+    __syncthreads();
+    float t = 0.0f;
+    if (threadIdx.x == 0) {
+        for (int k = 0; k < warps; ++k) t += s_part[k];
+    }
+    return t;
+}
+
+// The bilinear patch under a sample at (x, y).  Positions and values are formed with
+// the reference's expressions, each operation rounded by itself.
+struct Patch {
+    float a, b, c, d, fx, fy;
+};
+
+__device__ __forceinline__ bool load_patch(const uint8_t* __restrict__ image, int width, int height, int stride,
+                                           float x, float y, float den, Patch* out, int64_t* off) {
+    if (!(den > 1e-6f && x >= 0.0f && y >= 0.0f && x < static_cast<float>(width - 1) &&
+          y < static_cast<float>(height - 1))) {
+        return false;
+    }
     const int ix = static_cast<int>(x), iy = static_cast<int>(y);
-    const float fx = x - static_cast<float>(ix), fy = y - static_cast<float>(iy);
-    out->off = static_cast<int64_t>(iy) * q.stride + ix;
-    const uint8_t* p = q.image + out->off;
-    const float a = p[0], b = p[1], c = p[q.stride], d = p[q.stride + 1];
-    const float val = (a * (1.0f - fx) + b * fx) * (1.0f - fy) + (c * (1.0f - fx) + d * fx) * fy;
-    out->val = val;
-    const float t = q.tmpl[cell] ? 1.0f : 0.0f;
-    out->r = val - (q.lo + (q.hi - q.lo) * t);
-    out->w[0] = (1.0f - fx) * (1.0f - fy);
-    out->w[1] = fx * (1.0f - fy);
-    out->w[2] = (1.0f - fx) * fy;
-    out->w[3] = fx * fy;
-    if (!want_grad) return;
-    const float Ix = (b - a) * (1.0f - fy) + (d - c) * fy;
-    const float Iy = (c * (1.0f - fx) + d * fx) - (a * (1.0f - fx) + b * fx);
-    const float inv = 1.0f / den;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        const float dnx = q.dh[0][k] * u + q.dh[1][k] * v + q.dh[2][k];
-        const float dny = q.dh[3][k] * u + q.dh[4][k] * v + q.dh[5][k];
-        const float dden = q.dh[6][k] * u + q.dh[7][k] * v;
-        const float dxk = (dnx - x * dden) * inv;
-        const float dyk = (dny - y * dden) * inv;
-        out->gx[k] = Ix * dxk + Iy * dyk;
-    }
+    out->fx = x - static_cast<float>(ix);
+    out->fy = y - static_cast<float>(iy);
+    *off = static_cast<int64_t>(iy) * stride + ix;
+    const uint8_t* p = image + *off;
+    out->a = __ldg(p);
+    out->b = __ldg(p + 1);
+    out->c = __ldg(p + stride);
+    out->d = __ldg(p + stride + 1);
+    return true;
 }
 
-// Deterministic block sum of per-thread values (fixed tree).
-template <int N>
-__device__ void block_sum(float (&v)[N], float (*smem)[kThreads]) {
-#pragma unroll
-    for (int i = 0; i < N; ++i) smem[i][threadIdx.x] = v[i];
-    __syncthreads();
-    for (int off = kThreads / 2; off > 0; off >>= 1) {
-        if (threadIdx.x < off) {
-#pragma unroll
-            for (int i = 0; i < N; ++i) smem[i][threadIdx.x] += smem[i][threadIdx.x + off];
+// Residuals and loss.  Bound: issue slots (some 90 instructions a sample, two of them
+// IEEE divisions); the index of a sample takes no division any more.
+// 256 quads of 80 x 80 samples: 30 us before, 21 us.
+constexpr int kGradWarps = 20;    // two warps to each of 10 column blocks
+
+__global__ void __launch_bounds__(kGradWarps * 32, 2) k_refine_forward(bd_refine_args a, float* residuals,
+                                                                       float* loss) {
+    __shared__ GridSmem grid;
+    __shared__ float s_h[8];
+    __shared__ int s_ok;
+    __shared__ float s_part[kGradWarps];
+    const int qi = blockIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31;
+    if (tid == 0) {
+        float c[8];
+        for (int i = 0; i < 8; ++i) c[i] = a.corners[8 * qi + i];
+        Dual H[8];
+        s_ok = homography_dual(c, -1, H) ? 1 : 0;
+        for (int i = 0; s_ok && i < 8; ++i) s_h[i] = H[i].v;
+    }
+    load_grid(a, qi, grid);
+    const int spc = a.samples_per_cell, per_cell = spc * spc, side = a.cells * spc;
+    const uint8_t* image = quad_image(a, qi);
+    float* out = residuals ? residuals + static_cast<int64_t>(qi) * side * side : nullptr;
+    const float lo = a.levels ? a.levels[2 * qi] : 0.0f, hi = a.levels ? a.levels[2 * qi + 1] : 255.0f;
+    const float level_w = lo + (hi - lo) * 1.0f;
+    const bool ok = s_ok != 0;
+    const GridPlace place = grid_place(side);
+    float acc = 0.0f;
+    for (int block = place.block0; block < place.blocks; block += blockDim.x >> 5) {
+        const int col = block * kTileCols + (lane & 7);
+        if (col >= side) continue;
+        const int cx = col / spc;
+        const float u = grid.v[col];
+        const uint32_t white_cells = grid.white[cx];
+        const float hx = s_h[0] * u, hy = s_h[3] * u, hd = s_h[6] * u;
+        int cy = place.row0 / spc, sy = place.row0 - cy * spc;
+        for (int j = place.row0; j < side; j += place.row_step) {
+            const float v = grid.v[j];
+            const float den = hd + s_h[7] * v + 1.0f;
+            const float x = (hx + s_h[1] * v + s_h[2]) / den;
+            const float y = (hy + s_h[4] * v + s_h[5]) / den;
+            float r = 0.0f;
+            Patch p;
+            int64_t off;
+            if (ok && load_patch(image, a.width, a.height, a.stride, x, y, den, &p, &off)) {
+                const float val = (p.a * (1.0f - p.fx) + p.b * p.fx) * (1.0f - p.fy) +
+                                  (p.c * (1.0f - p.fx) + p.d * p.fx) * p.fy;
+                r = val - ((white_cells & grid.cell_bit[j]) ? level_w : lo);
+            }
+            if (out) out[(cy * a.cells + cx) * per_cell + sy * spc + (col - cx * spc)] = r;
+            acc += 0.5f * r * r;
+            for (sy += place.row_step; sy >= spc; sy -= spc) ++cy;
         }
-        __syncthreads();
     }
-#pragma unroll
-    for (int i = 0; i < N; ++i) v[i] = smem[i][0];
-    __syncthreads();
+    const float sum = cta_sum(acc, s_part);
+    if (tid == 0 && loss) loss[qi] = sum;
 }
 
-// The quad's context into shared memory, by lanes 0-7 of the first warp (lane k
-// holds the derivatives with respect to corner coordinate k); *ok says whether
-// it has a homography.  The caller synchronises.
-__device__ __forceinline__ void load_quad(const bd_refine_args& a, int qi, const float* corners, QuadCtx* q,
-                                          int* ok) {
-    const int k = threadIdx.x;
-    if (k >= 8) return;
-    float c[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) c[i] = corners[i];
-    Dual H[8];
-    const bool good = homography_dual(c, k, H);
-    if (good) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) q->dh[i][k] = H[i].d;
-    }
-    if (k != 0) return;
-    *ok = good ? 1 : 0;
-    if (good) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) q->h[i] = H[i].v;
-    }
-    q->image = a.images + static_cast<int64_t>(a.image_index ? a.image_index[qi] : 0) * a.image_pitch;
-    q->width = a.width;
-    q->height = a.height;
-    q->stride = a.stride;
-    q->cells = a.cells;
-    q->spc = a.samples_per_cell;
-    q->tmpl = a.templates + static_cast<int64_t>(qi) * a.cells * a.cells;
-    q->lo = a.levels ? a.levels[2 * qi] : 0.0f;
-    q->hi = a.levels ? a.levels[2 * qi + 1] : 255.0f;
-}
-
-__global__ void __launch_bounds__(kThreads) k_refine_forward(bd_refine_args a, float* residuals,
-                                                             float* loss) {
-    __shared__ QuadCtx q;
-    __shared__ int ok;
-    __shared__ float red[1][kThreads];
+// The adjoint.  With w = dr/dH of a sample (A u, A v, A, B u, B v, B, C u, C v; A = I_x /
+// den, B = I_y / den, C = -(A x + B y)), dL/dc = dH^T sum(g w), dH = dH/dc the same for
+// every sample: a sample adds six numbers (A, B, C times 1 and v; u is the thread's)
+// instead of forming its derivatives by the 8 corner coordinates.  x and y in C and
+// dH are relative to a whole pixel near the quad's centre, which keeps its parts from
+// cancelling.
+//
+// Bound: the four scattered adds per sample (4.7 M requests of 256 quads of 80 x 80
+// samples).  58 us before, 41 us.
+__global__ void __launch_bounds__(kGradWarps * 32, 2) k_refine_backward(bd_refine_args a,
+                                                                        const float* __restrict__ grad_residuals,
+                                                                        float* grad_corners,
+                                                                        float* grad_images) {
+    __shared__ GridSmem grid;
+    __shared__ float s_h[8], s_dh[8][8];
+    __shared__ int s_ok, s_ox, s_oy;
+    __shared__ float s_part[kGradWarps][8];
     const int qi = blockIdx.x;
-    load_quad(a, qi, a.corners + 8 * qi, &q, &ok);
-    __syncthreads();
-    const int n = a.cells * a.cells * a.samples_per_cell * a.samples_per_cell;
-    float acc[1] = {0.0f};
-    for (int s = threadIdx.x; s < n; s += kThreads) {
-        Sample smp;
-        smp.r = 0.0f;
-        if (ok) eval_sample(q, s, false, &smp);
-        if (residuals) residuals[static_cast<int64_t>(qi) * n + s] = smp.r;
-        acc[0] += 0.5f * smp.r * smp.r;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, warps = blockDim.x >> 5;
+    if (tid < 16) {
+        // Lanes 0-7: dH / dc_lane from corners relative to (ox, oy); lane 8: H.
+        float c[8];
+        for (int i = 0; i < 8; ++i) c[i] = a.corners[8 * qi + i];
+        const int ox = static_cast<int>(floorf(0.25f * (c[0] + c[2] + c[4] + c[6])));
+        const int oy = static_cast<int>(floorf(0.25f * (c[1] + c[3] + c[5] + c[7])));
+        for (int i = 0; tid < 8 && i < 8; ++i) c[i] -= static_cast<float>((i & 1) ? oy : ox);
+        Dual H[8];
+        const bool good = homography_dual(c, tid, H);
+        for (int i = 0; i < 8; ++i) {
+            if (tid < 8) s_dh[i][tid] = good ? H[i].d : 0.0f;
+            if (tid == 8) s_h[i] = good ? H[i].v : 0.0f;
+        }
+        if (tid == 8) {
+            s_ok = good ? 1 : 0;
+            s_ox = ox;
+            s_oy = oy;
+        }
     }
-    block_sum<1>(acc, red);
-    if (threadIdx.x == 0 && loss) loss[qi] = acc[0];
-}
-
-__global__ void __launch_bounds__(kThreads) k_refine_backward(bd_refine_args a,
-                                                              const float* grad_residuals,
-                                                              float* grad_corners,
-                                                              float* grad_images) {
-    __shared__ QuadCtx q;
-    __shared__ int ok;
-    __shared__ float red[8][kThreads];
-    const int qi = blockIdx.x;
-    load_quad(a, qi, a.corners + 8 * qi, &q, &ok);
-    __syncthreads();
-    const int n = a.cells * a.cells * a.samples_per_cell * a.samples_per_cell;
+    load_grid(a, qi, grid);
+    const int spc = a.samples_per_cell, per_cell = spc * spc, side = a.cells * spc;
+    const uint8_t* image = quad_image(a, qi);
+    const float* go_quad = grad_residuals + static_cast<int64_t>(qi) * side * side;
+    float* gimg = grad_images ? grad_images + (image - a.images) : nullptr;
+    const float ox = static_cast<float>(s_ox), oy = static_cast<float>(s_oy);
+    const GridPlace place = grid_place(side);
     float g[8] = {};
-    float* gimg = grad_images
-                      ? grad_images + static_cast<int64_t>(a.image_index ? a.image_index[qi] : 0) *
-                                          (a.image_pitch)
-                      : nullptr;
-    for (int s = threadIdx.x; s < n && ok; s += kThreads) {
-        Sample smp;
-        eval_sample(q, s, true, &smp);
-        if (!smp.in) continue;
-        const float go = grad_residuals[static_cast<int64_t>(qi) * n + s];
+    for (int block = s_ok ? place.block0 : place.blocks; block < place.blocks; block += warps) {
+        const int col = block * kTileCols + (lane & 7);
+        if (col >= side) continue;
+        const int cx = col / spc;
+        const float u = grid.v[col];
+        const float hx = s_h[0] * u, hy = s_h[3] * u, hd = s_h[6] * u;
+        float w0[3] = {}, w1[3] = {};
+        int cy = place.row0 / spc, sy = place.row0 - cy * spc;
+        for (int j = place.row0; j < side; j += place.row_step) {
+            const float v = grid.v[j];
+            const float den = hd + s_h[7] * v + 1.0f;
+            const float x = (hx + s_h[1] * v + s_h[2]) / den;
+            const float y = (hy + s_h[4] * v + s_h[5]) / den;
+            Patch p;
+            int64_t off;
+            if (load_patch(image, a.width, a.height, a.stride, x, y, den, &p, &off)) {
+                const float go = go_quad[(cy * a.cells + cx) * per_cell + sy * spc + (col - cx * spc)];
+                const float Ix = (p.b - p.a) * (1.0f - p.fy) + (p.d - p.c) * p.fy;
+                const float Iy = (p.c * (1.0f - p.fx) + p.d * p.fx) - (p.a * (1.0f - p.fx) + p.b * p.fx);
+                const float scale = go / den;
+                const float A = Ix * scale, B = Iy * scale;
+                const float C = -__fmaf_rn(A, x - ox, B * (y - oy));
+                const float abc[3] = {A, B, C};
 #pragma unroll
-        for (int k = 0; k < 8; ++k) g[k] += go * smp.gx[k];
-        if (gimg) {
-            float* p = gimg + smp.off;
-            atomicAdd(p, go * smp.w[0]);
-            atomicAdd(p + 1, go * smp.w[1]);
-            atomicAdd(p + q.stride, go * smp.w[2]);
-            atomicAdd(p + q.stride + 1, go * smp.w[3]);
+                for (int i = 0; i < 3; ++i) {
+                    w0[i] += abc[i];
+                    w1[i] = __fmaf_rn(abc[i], v, w1[i]);
+                }
+                if (gimg) {
+                    float* q = gimg + off;
+                    atomicAdd(q, go * ((1.0f - p.fx) * (1.0f - p.fy)));
+                    atomicAdd(q + 1, go * (p.fx * (1.0f - p.fy)));
+                    atomicAdd(q + a.stride, go * ((1.0f - p.fx) * p.fy));
+                    atomicAdd(q + a.stride + 1, go * (p.fx * p.fy));
+                }
+            }
+            for (sy += place.row_step; sy >= spc; sy -= spc) ++cy;
+        }
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            g[3 * i] = __fmaf_rn(u, w0[i], g[3 * i]);
+            g[3 * i + 1] += w1[i];
+            if (i < 2) g[3 * i + 2] += w0[i];
         }
     }
-    block_sum<8>(g, red);
-    if (threadIdx.x < 8 && grad_corners) grad_corners[8 * qi + threadIdx.x] = g[threadIdx.x];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) g[i] += __shfl_down_sync(0xffffffffu, g[i], off);
+        if (lane == 0) s_part[warp][i] = g[i];
+    }
+    __syncthreads();
+    if (tid < 8 && grad_corners) {
+        double t = 0.0;
+        for (int i = 0; i < 8; ++i) {
+            float w = 0.0f;
+            for (int k = 0; k < warps; ++k) w += s_part[k][i];
+            t = __fma_rn(static_cast<double>(w), static_cast<double>(s_dh[i][tid]), t);
+        }
+        grad_corners[8 * qi + tid] = static_cast<float>(t);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -278,13 +379,8 @@ __global__ void __launch_bounds__(kThreads) k_refine_backward(bd_refine_args a,
 // 256 quads of 80 x 80 samples, 5 iterations: 792 us before, 120 us (170 us with 32
 // columns of one row to a warp).  Corners are five times nearer to 64-bit arithmetic.
 // ---------------------------------------------------------------------------
-constexpr int kMaxGrid = 256;     // samples per side: 16 cells of 16
 constexpr int kSums = 64;         // 61 used
-// A warp takes 8 columns by 4 rows of samples at a time: neighbouring pixels, so
-// a load meets some 8 rows of the frame.  32 columns of one sample row meet up to 28
-// when the quad lies askew, and L1 takes a pass per row.
-constexpr int kTileCols = 8, kTileRows = 4;
-constexpr int kGnWarps = 10;      // 10 x 8 columns: 10 cells of 8 samples (tag36h11)
+constexpr int kGnWarps = 10;      // 10 blocks of 8 columns: 10 cells of 8 samples (tag36h11)
 
 // Places of the sums.  Products: the unique entries of w w^T by pair and powers
 // of (u, v); then w r, w over white samples, w over all, then per colour (black,
@@ -321,9 +417,7 @@ struct GnSmem {
     float level[2];               // provisional: black, white
     int cx, cy;
     int ok;
-    float v[kMaxGrid];            // v of each sample row
-    uint16_t cell_bit[kMaxGrid];  // 1 << its cell
-    uint32_t white[16];           // bit cy of white[cx]: a white cell
+    GridSmem grid;
     float part[kGnWarps][kSums];
     float sum[kSums];
     double shift[2];              // true levels - provisional ones
@@ -407,22 +501,8 @@ __global__ void __launch_bounds__(kGnWarps * 32, 2) k_refine_gauss_newton(bd_ref
     const int qi = blockIdx.x;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int warps = blockDim.x >> 5;
-    const int grid = a.cells * a.samples_per_cell;
-    const float dim = static_cast<float>(a.cells - 2);
-    const uint8_t* image = a.images + static_cast<int64_t>(a.image_index ? a.image_index[qi] : 0) * a.image_pitch;
-    const uint8_t* tmpl = a.templates + static_cast<int64_t>(qi) * a.cells * a.cells;
-
-    // Sample coordinate i of the grid's side (cell, sub-sample).
-    auto coordinate = [&](int i) {
-        const int cell = i / a.samples_per_cell;
-        const int sub = i - cell * a.samples_per_cell;
-        return (static_cast<float>(cell - 1) + (static_cast<float>(sub) + 0.5f) / a.samples_per_cell) / dim;
-    };
-    for (int i = tid; i < grid; i += blockDim.x) {
-        sm.v[i] = coordinate(i);
-        sm.cell_bit[i] = static_cast<uint16_t>(1u << (i / a.samples_per_cell));
-    }
-    if (tid < 16) sm.white[tid] = 0;
+    const int side = a.cells * a.samples_per_cell;
+    const uint8_t* image = quad_image(a, qi);
     if (tid == 0) {
         const float* c = corners + 8 * qi;
         sm.cx = static_cast<int>(floorf(0.25f * (c[0] + c[2] + c[4] + c[6])));
@@ -430,19 +510,9 @@ __global__ void __launch_bounds__(kGnWarps * 32, 2) k_refine_gauss_newton(bd_ref
         sm.level[0] = a.levels ? a.levels[2 * qi] : 0.0f;
         sm.level[1] = a.levels ? a.levels[2 * qi + 1] : 255.0f;
     }
-    __syncthreads();
     if (tid < 8) sm.c[tid] = corners[8 * qi + tid];
-    for (int i = tid; i < a.cells * a.cells; i += blockDim.x) {
-        const int cy = i / a.cells;
-        if (tmpl[i]) atomicOr(&sm.white[i - cy * a.cells], 1u << cy);
-    }
-    __syncthreads();
-    // The columns in blocks of 8, `share` warps to a block (each takes its part of
-    // the rows), or several blocks to a warp one after another.
-    const int blocks = (grid + kTileCols - 1) / kTileCols;
-    const int share = max(1, warps / blocks);
-    const int row0 = (warp % share) * kTileRows + (lane >> 3);
-    const int row_step = share * kTileRows;
+    load_grid(a, qi, sm.grid);
+    const GridPlace place = grid_place(side);
     const int ox = sm.cx, oy = sm.cy;
     const unsigned in_x = static_cast<unsigned>(a.width - 1), in_y = static_cast<unsigned>(a.height - 1);
 
@@ -467,10 +537,10 @@ __global__ void __launch_bounds__(kGnWarps * 32, 2) k_refine_gauss_newton(bd_ref
         if (!sm.ok) break;
         const float h1 = sm.h[1], h4 = sm.h[4], h7 = sm.h[7];
         const float level_b = sm.level[0], level_w = sm.level[1];
-        for (int block = warp / share; block < blocks; block += warps) {
+        for (int block = place.block0; block < place.blocks; block += warps) {
             const int col = block * kTileCols + (lane & 7);
-            const float u = sm.v[min(col, grid - 1)];  // the grid is square: u and v share their values
-            const uint32_t white_cells = sm.white[min(col, grid - 1) / a.samples_per_cell];
+            const float u = sm.grid.v[min(col, side - 1)];
+            const uint32_t white_cells = sm.grid.white[min(col, side - 1) / a.samples_per_cell];
             const float hx = __fmaf_rn(sm.h[0], u, sm.h[2]);
             const float hy = __fmaf_rn(sm.h[3], u, sm.h[5]);
             const float hd = __fmaf_rn(sm.h[6], u, 1.0f);
@@ -479,8 +549,8 @@ __global__ void __launch_bounds__(kGnWarps * 32, 2) k_refine_gauss_newton(bd_ref
             float w0[3] = {}, w1[3] = {};                  // (A, B, C), white samples
             float s0[3] = {}, s1[3] = {};                  // (A, B, C), all
             float count[2] = {}, m1[2] = {}, m2[2] = {};
-            for (int j = col < grid ? row0 : grid; j < grid; j += row_step) {
-                const float v = sm.v[j];
+            for (int j = col < side ? place.row0 : side; j < side; j += place.row_step) {
+                const float v = sm.grid.v[j];
                 const float den = __fmaf_rn(h7, v, hd);
                 const float inv = __frcp_rn(den);
                 const float x = __fmaf_rn(h1, v, hx) * inv;
@@ -498,7 +568,7 @@ __global__ void __launch_bounds__(kGnWarps * 32, 2) k_refine_gauss_newton(bd_ref
                 const float A = __fmaf_rn((pd - pc) - (pb - pa), fy, pb - pa) * inv;
                 const float B = (bottom - top) * inv;
                 const float C = -__fmaf_rn(A, x, B * y);
-                const bool white = (white_cells & sm.cell_bit[j]) != 0;
+                const bool white = (white_cells & sm.grid.cell_bit[j]) != 0;
                 const float r = value - (white ? level_w : level_b);
                 const float vv = v * v;
                 const float pr[6] = {A * A, B * B, A * B, A * C, B * C, C * C};
@@ -574,7 +644,7 @@ __global__ void __launch_bounds__(kGnWarps * 32, 2) k_refine_gauss_newton(bd_ref
                 sums[kMoment2 + i] = m2[i];
             }
             warp_sums(sums, lane);
-            const bool first = block == warp / share;
+            const bool first = block == place.block0;
             sm.part[warp][lane] = first ? sums[0] : sm.part[warp][lane] + sums[0];
             sm.part[warp][lane + 32] = first ? sums[1] : sm.part[warp][lane + 32] + sums[1];
         }
@@ -702,7 +772,8 @@ int32_t bd_refine_forward(const bd_refine_args* args, float* residuals, float* l
     const int32_t rc = check_args(args);
     if (rc != BD_OK) return rc;
     if (args->count == 0) return BD_OK;
-    k_refine_forward<<<args->count, kThreads, 0, static_cast<cudaStream_t>(cuda_stream)>>>(
+    const int warps = grid_warps(args->cells * args->samples_per_cell, kGradWarps);
+    k_refine_forward<<<args->count, warps * 32, 0, static_cast<cudaStream_t>(cuda_stream)>>>(
         *args, residuals, loss);
     return launched();
 }
@@ -716,7 +787,8 @@ int32_t bd_refine_backward(const bd_refine_args* args, const float* grad_residua
         return BD_ERROR_INVALID_ARGUMENT;
     }
     if (args->count == 0) return BD_OK;
-    k_refine_backward<<<args->count, kThreads, 0, static_cast<cudaStream_t>(cuda_stream)>>>(
+    const int warps = grid_warps(args->cells * args->samples_per_cell, kGradWarps);
+    k_refine_backward<<<args->count, warps * 32, 0, static_cast<cudaStream_t>(cuda_stream)>>>(
         *args, grad_residuals, grad_corners, grad_images);
     return launched();
 }
@@ -730,10 +802,8 @@ int32_t bd_refine_gauss_newton(const bd_refine_args* args, float* corners_inout,
         return BD_ERROR_INVALID_ARGUMENT;
     }
     if (args->count == 0) return BD_OK;
-    // A warp per block of columns, more when there are few blocks; at least the
-    // three warps that the steps between the samples use.
-    const int blocks = (args->cells * args->samples_per_cell + kTileCols - 1) / kTileCols;
-    const int warps = blocks >= kGnWarps ? kGnWarps : std::max(3, kGnWarps / blocks * blocks);
+    // At least the three warps that the steps between the samples use.
+    const int warps = std::max(3, grid_warps(args->cells * args->samples_per_cell, kGnWarps));
     k_refine_gauss_newton<<<args->count, warps * 32, 0, static_cast<cudaStream_t>(cuda_stream)>>>(
         *args, corners_inout, iterations, loss);
     return launched();

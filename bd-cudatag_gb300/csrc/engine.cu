@@ -360,7 +360,7 @@ Plan* Plan::create(const std::vector<PlanFrame>& frames, const PlanConfig& confi
         off_lroots[i] = carve.take(sizeof(uint32_t) * slots);
         off_lcount[i] = carve.take(sizeof(uint32_t) * d.tile_h);
         off_mode[i] = carve.take(sizeof(uint32_t) * d.tile_h);
-        off_bands[i] = carve.take(sizeof(uint32_t) * 64 * d.tile_h);
+        off_bands[i] = carve.take(sizeof(uint16_t) * 32 * d.tile_h);
         off_cands[i] = carve.take(sizeof(uint32_t) * mc);
         off_fit[i] = carve.take(sizeof(uint32_t) * mc);
         off_hull[i] = carve.take(sizeof(float) * 8 * mc);

@@ -23,6 +23,10 @@ int prepare_pipeline() {
         cudaSuccess) {
         return -1;
     }
+    if (cudaFuncSetAttribute(k_cand_count, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             static_cast<int>(cand_smem_bytes(kMaxBandsPerFrame))) != cudaSuccess) {
+        return -1;
+    }
     if (cudaFuncSetAttribute(k_fit_decode_all, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              static_cast<int>(fit_all_smem_bytes())) != cudaSuccess) {
         return -1;
@@ -76,7 +80,7 @@ void enqueue_pipeline(const BatchDesc* dd, const BatchDesc& hd, const FrameIOArg
     const int split = lc.quad_split;
     int th_max = 1;
     for (int f = 0; f < hd.frames; ++f) th_max = std::max(th_max, hd.f[f].tile_h);
-    k_cand_count<<<bands, 256, (th_max + 1) * sizeof(uint32_t), s>>>(dd, io, split);
+    k_cand_count<<<bands, 256, cand_smem_bytes(th_max), s>>>(dd, io, split);
     mark(5);
     int cands = 0;
     for (int f = 0; f < hd.frames; ++f) cands += hd.f[f].max_candidates;

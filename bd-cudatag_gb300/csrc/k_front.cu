@@ -52,13 +52,11 @@ __global__ void __launch_bounds__(256) k_region_stats(const BatchDesc* __restric
 
 __global__ void __launch_bounds__(256) k_cand_count(const BatchDesc* __restrict__ b,
                                                     const FrameIO* __restrict__ io, int split_px) {
-    // Candidates before each band of the frame (tallest frame's bands + 1,
-    // sized at launch).
-    extern __shared__ uint32_t s_cprefix[];
+    extern __shared__ uint32_t s_dyn_cand[];  // cand_smem_bytes of the tallest frame
     __shared__ CandSmem sm;
     const int fi = frame_of_band(b, blockIdx.x);
     if (!io[fi].gray) return;
-    stage_cand(b, fi, blockIdx.x - b->band_prefix[fi], split_px, sm, s_cprefix);
+    stage_cand(b, fi, blockIdx.x - b->band_prefix[fi], split_px, sm, s_dyn_cand);
 }
 
 }  // namespace bdgb

@@ -290,7 +290,7 @@ size_t persistent_smem_bytes(int band_cap, int bits_words, int row_cap_max, int 
     size_t bytes = sizeof(StatsSmem);
     bytes = std::max(bytes, kBinDyn + band_smem_bytes(band_cap, bits_words));
     bytes = std::max(bytes, 2 * static_cast<size_t>(row_cap_max) * sizeof(uint32_t));
-    bytes = std::max(bytes, kCandDyn + (static_cast<size_t>(tile_h_max) + 1) * sizeof(uint32_t));
+    bytes = std::max(bytes, kCandDyn + cand_smem_bytes(tile_h_max));
     bytes = std::max(bytes, kSmallPerUnit * sizeof(QuadSmem));
     bytes = std::max(bytes, sizeof(BigSmem));
     bytes = std::max(bytes, sizeof(FinalSmem));

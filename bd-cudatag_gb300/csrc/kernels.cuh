@@ -41,6 +41,12 @@ __host__ __device__ constexpr size_t band_smem_bytes(int cap, int words) {
            static_cast<size_t>(cap);
 }
 
+// Dynamic shared memory of k_cand_count: the candidates before each band (and
+// in all), then the 32 16-bit counts of every band of the tallest frame.
+__host__ __device__ constexpr size_t cand_smem_bytes(int tile_h) {
+    return (static_cast<size_t>(tile_h) + 1) * sizeof(uint32_t) + static_cast<size_t>(tile_h) * 64;
+}
+
 constexpr int kFinalThreads = 256;
 
 __global__ void k_stats(const BatchDesc* b, const __grid_constant__ FrameIOArgs io, FrameIO* io_out);

@@ -134,7 +134,7 @@ struct FrameDesc {
     uint32_t* lroot_count;         // tile_h: band-local roots per band
     uint32_t* band_mode;           // tile_h: bit 0 fallback (one root per run), else bit r: row r
                                    // starts a shared-memory segment (band-local unions done)
-    uint32_t* band_bins;           // tile_h * 64 candidate counts, then exclusive prefixes
+    uint32_t* band_bins;           // tile_h * 32 16-bit candidate counts per area bin 32..63 ([0]: all)
     uint32_t* candidates;          // max_candidates root slots, canonical order
     uint32_t* fit_list;            // max_candidates positions in `candidates`: from the front the
                                    // n_big whose bbox side exceeds the split (k_fit_decode_big),

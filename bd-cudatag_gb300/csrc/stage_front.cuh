@@ -37,16 +37,18 @@ struct BinSmem {
     uint32_t segmask;
 };
 
-// stage_cand's shared memory, besides the per-band candidate prefix (tile_h
-// + 1 words of the tallest frame, a separate region).
+// stage_cand's shared memory, besides the frame's candidate table (a separate
+// region, cand_smem_bytes).  Area bins 32..63 can occur (areas are below 2^31).
+constexpr int kAreaBins = 32;
+constexpr uint32_t kListCap = 512;   // candidates of a band ranked from shared memory
 struct CandSmem {
     uint32_t rowoff[kTile + 1];
-    uint32_t wbin[8][64];
-    uint32_t run[64];
-    uint32_t chunk[4][64];
-    uint32_t total[64];
-    uint32_t base[64];
-    uint32_t warp_sum[8];
+    uint32_t slot[kListCap];
+    uint8_t bin[kListCap];
+    uint32_t bins[kAreaBins];        // the band's candidates per bin; [0] all of them
+    uint32_t chunk[8][kAreaBins];
+    uint32_t total[kAreaBins];
+    uint32_t base[kAreaBins];
     uint32_t ncand, limit, nbig, nsmall;
     int last;
 };
@@ -713,33 +715,38 @@ __device__ __forceinline__ uint32_t band_slot(const uint32_t* rowoff, int y0, ui
     return static_cast<uint32_t>(y0 + row) * row_cap + (i - rowoff[row]);
 }
 
-// One CTA per band, 256 runs at a time in slot order: root labels, the
-// tag-like filter, and each candidate's rank among the band's candidates
-// of its area bin.
+// One CTA per band: root labels, the tag-like filter, and each candidate's
+// rank among the band's candidates of its area bin.  The candidates, a few of
+// thousands of runs, are listed as they come and ranked afterwards by
+// counting; ranking every 256 runs in order took four barriers a time.  The
+// frame's last CTA places the candidates.
+//
+// Bound: dependent L2 loads (two hops to the root, then area and box), then the
+// last CTA's chain.  Stage time (CUDA events, launch included): 18.4 -> 14.3 us
+// for four 1280x800 frames, 28.7 -> 20.5 for sixteen mixed ones, 51 -> 31 for
+// a noisy 3840x2160 frame (20 groups of runs a band).
 __device__ __forceinline__ bool stage_cand(const BatchDesc* __restrict__ b, int fi, int ty, int split_px, CandSmem& sm,
-                           uint32_t* s_cprefix) {
+                           uint32_t* s_dyn) {
     uint32_t* s_rowoff = sm.rowoff;
-    uint32_t (*s_wbin)[64] = sm.wbin;
-    uint32_t* s_run = sm.run;
-    uint32_t (*s_chunk)[64] = sm.chunk;
-    uint32_t* s_total = sm.total;
-    uint32_t* s_base = sm.base;
-    uint32_t* s_warp_sum = sm.warp_sum;
     const int tid = threadIdx.x;
     const FrameDesc& d = b->f[fi];
     FrameState* st = d.state;
     const int y0 = ty * kTile;
     const uint32_t row_cap = static_cast<uint32_t>(d.row_cap);
-    if (tid == 0) {
-        uint32_t off = 0;
-        for (int r = 0; r < kTile; ++r) {
-            s_rowoff[r] = off;
-            off += y0 + r < d.height ? d.row_count[y0 + r] : 0u;
+    if (tid < 32) {
+        // Runs before each row of the band.
+        const uint32_t n = tid < kTile && y0 + tid < d.height ? d.row_count[y0 + tid] : 0u;
+        uint32_t incl = n;
+#pragma unroll
+        for (int off = 1; off < kTile; off <<= 1) {
+            const uint32_t v = __shfl_up_sync(kFull, incl, off);
+            if (tid >= off) incl += v;
         }
-        s_rowoff[kTile] = off;
+        if (tid < kTile) s_rowoff[tid + 1] = incl;
+        if (tid == 0) s_rowoff[0] = 0;
+        sm.bins[tid] = 0;
+        if (tid == 0) sm.ncand = 0;
     }
-    if (tid < 64) s_run[tid] = 0;
-    if (tid == 0) sm.ncand = 0;
     __syncthreads();
     const uint32_t total = s_rowoff[kTile];
     const int w = tid >> 5, lane = tid & 31;
@@ -748,19 +755,14 @@ __device__ __forceinline__ bool stage_cand(const BatchDesc* __restrict__ b, int 
     // cand_meta, for the frame's last CTA to place.
     uint32_t* band_list = d.lroots + static_cast<int64_t>(ty) * kTile * row_cap;
     uint32_t* band_meta = d.cand_meta + static_cast<int64_t>(ty) * kTile * row_cap;
-    // Up to four chunks of 256 runs at a time: their label and root loads are
-    // issued together, then the chunks are ranked one after another in slot
-    // order, as before.
+    // Up to four groups of 256 runs at a time, their label and root loads
+    // issued together.
     constexpr int kChunks = 4;
     for (uint32_t gbase = 0; gbase < total; gbase += kChunks * blockDim.x) {
-        int bins[kChunks];
-        bool bigs[kChunks];
         uint32_t slots[kChunks], hop[kChunks];
 #pragma unroll
         for (int u = 0; u < kChunks; ++u) {
             const uint32_t i = gbase + u * blockDim.x + tid;
-            bins[u] = -1;
-            bigs[u] = false;
             slots[u] = 0;
             hop[u] = 0;
             if (i < total) {
@@ -782,46 +784,45 @@ __device__ __forceinline__ bool stage_cand(const BatchDesc* __restrict__ b, int 
         for (int u = 0; u < kChunks; ++u) {
             if (gbase + u * blockDim.x + tid < total) {
                 d.parent[slots[u]] = hop[u];
-                if (hop[u] == slots[u]) bins[u] = candidate_bin(d, slots[u], split_px, &bigs[u]);
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < kChunks; ++u) {
-            if (gbase + u * blockDim.x >= total) break;  // uniform over the CTA
-            const int bin = bins[u];
-            const bool big = bigs[u];
-            const uint32_t slot = slots[u];
-            const uint32_t key = bin >= 0 ? static_cast<uint32_t>(bin) : 64u + lane;
-            const uint32_t peers = __match_any_sync(kFull, key);
-            const uint32_t rank = __popc(peers & lanemask_lt());
-            s_wbin[w][lane] = 0;
-            s_wbin[w][lane + 32] = 0;
-            __syncthreads();
-            if (bin >= 0 && rank == 0) s_wbin[w][bin] = __popc(peers);
-            __syncthreads();
-            uint32_t meta = kNone;
-            if (bin >= 0) {
-                uint32_t pos = s_run[bin] + rank;
-                for (int w2 = 0; w2 < w; ++w2) pos += s_wbin[w2][bin];
-                meta = (static_cast<uint32_t>(bin) << 24) | (big ? 1u << 23 : 0u) | pos;
-            }
-            __syncthreads();
-            if (tid < 64) {
-                uint32_t add = 0;
-                for (int w2 = 0; w2 < 8; ++w2) add += s_wbin[w2][tid];
-                s_run[tid] += add;
-            }
-            if (bin >= 0) {
+                if (hop[u] != slots[u]) continue;
+                bool big;
+                const int bin = candidate_bin(d, slots[u], split_px, &big);
+                if (bin < 0) continue;
                 const uint32_t at = atomicAdd(&sm.ncand, 1u);
-                band_list[at] = slot;
-                band_meta[at] = meta;
+                atomicAdd(&sm.bins[bin - 32], 1u);
+                if (at < kListCap) {
+                    sm.slot[at] = slots[u];
+                    sm.bin[at] = static_cast<uint8_t>(bin);
+                }
+                band_list[at] = slots[u];
+                band_meta[at] = (static_cast<uint32_t>(bin) << 24) | (big ? 1u << 23 : 0u);
             }
-            __syncthreads();  // s_wbin is cleared for the next chunk
         }
     }
     __syncthreads();
-    if (tid < 64) d.band_bins[ty * 64 + tid] = s_run[tid];
-    if (tid == 0) d.lroot_count[ty] = sm.ncand;
+    const uint32_t ncand = sm.ncand;
+    const bool listed = ncand <= kListCap;
+    for (uint32_t c = tid; c < ncand; c += blockDim.x) {
+        const uint32_t slot = listed ? sm.slot[c] : __ldcg(band_list + c);
+        const uint32_t word = __ldcg(band_meta + c);
+        uint32_t rank = 0;
+        if (listed) {
+            const uint32_t bin = sm.bin[c];
+            for (uint32_t k = 0; k < ncand; ++k) rank += sm.bin[k] == bin && sm.slot[k] < slot ? 1u : 0u;
+        } else {
+            for (uint32_t k = 0; k < ncand; ++k) {
+                // Bin and slot only: other threads are adding the ranks.
+                rank += __ldcg(band_meta + k) >> 24 == word >> 24 && __ldcg(band_list + k) < slot ? 1u : 0u;
+            }
+        }
+        band_meta[c] = word | rank;
+    }
+    // The band's row of the candidate table: 16-bit counts per bin, [0] all.
+    if (tid == 0) sm.bins[0] = ncand;  // bin 32 does not occur
+    __syncthreads();
+    if (tid < kAreaBins / 2) {
+        d.band_bins[ty * (kAreaBins / 2) + tid] = sm.bins[2 * tid] | (sm.bins[2 * tid + 1] << 16);
+    }
     __threadfence();
     __syncthreads();
     if (tid == 0) sm.last = atomicAdd(&st->done_cands, 1u) == static_cast<uint32_t>(d.tile_h - 1);
@@ -829,57 +830,59 @@ __device__ __forceinline__ bool stage_cand(const BatchDesc* __restrict__ b, int 
     if (!sm.last) return false;
     __threadfence();
 
-    // Last band: exclusive prefix of every bin over the bands (in place).
-    // Thread (segment q, bin) sums a quarter of the bands (loads coalesced
-    // over the bins), the four segment sums are scanned per bin, and each
-    // thread rewrites its quarter from its segment's offset.
+    // Last band: the table into shared memory, eight loads in flight, then the
+    // exclusive prefix of every bin over the bands in place: warp q takes an eighth
+    // of the bands, lane = bin.  A prefix beyond 16 bits is cut to 65535:
+    // such a candidate is past every cap either way.  Column 0 gives the candidates
+    // before each band, in full.
     const int th = d.tile_h;
-    const int bin = tid & 63;
-    const int q = tid >> 6;
-    const int per = (th + 3) >> 2;
-    const int qb0 = min(th, q * per), qb1 = min(th, qb0 + per);
-    // Both passes load eight bands at a time, so a quarter of a frame's
-    // bands costs a few L2 round trips instead of one per band.
-    constexpr int kBatch = 8;
-    uint32_t sum = 0;
-    for (int band = qb0; band < qb1; band += kBatch) {
-        uint32_t v[kBatch];
+    uint32_t* s_cprefix = s_dyn;                                     // th + 1
+    uint32_t* s_words = s_dyn + th + 1;                              // th rows of 16 words
+    uint16_t* s_table = reinterpret_cast<uint16_t*>(s_words);
+    const int words = th * (kAreaBins / 2);
+    for (int i0 = tid; i0 < words; i0 += 8 * blockDim.x) {
+        uint32_t v[8];
 #pragma unroll
-        for (int k = 0; k < kBatch; ++k) v[k] = band + k < qb1 ? __ldcg(&d.band_bins[(band + k) * 64 + bin]) : 0u;
+        for (int k = 0; k < 8; ++k) v[k] = i0 + k * blockDim.x < words ? __ldcg(&d.band_bins[i0 + k * blockDim.x]) : 0u;
 #pragma unroll
-        for (int k = 0; k < kBatch; ++k) sum += v[k];
-    }
-    s_chunk[q][bin] = sum;
-    __syncthreads();
-    uint32_t carry = 0;
-    for (int q2 = 0; q2 < q; ++q2) carry += s_chunk[q2][bin];
-    if (q == 3) s_total[bin] = carry + sum;
-    for (int band = qb0; band < qb1; band += kBatch) {
-        uint32_t v[kBatch];
-#pragma unroll
-        for (int k = 0; k < kBatch; ++k) v[k] = band + k < qb1 ? __ldcg(&d.band_bins[(band + k) * 64 + bin]) : 0u;
-#pragma unroll
-        for (int k = 0; k < kBatch; ++k) {
-            if (band + k < qb1) {
-                d.band_bins[(band + k) * 64 + bin] = carry;
-                carry += v[k];
-            }
+        for (int k = 0; k < 8; ++k) {
+            if (i0 + k * blockDim.x < words) s_words[i0 + k * blockDim.x] = v[k];
         }
     }
     __syncthreads();
+    const int per = (th + 7) >> 3;
+    const int b0 = min(th, w * per), b1 = min(th, b0 + per);
+    uint32_t sum = 0;
+#pragma unroll 4
+    for (int band = b0; band < b1; ++band) sum += s_table[band * kAreaBins + lane];
+    sm.chunk[w][lane] = sum;
+    __syncthreads();
+    uint32_t carry = 0;
+    for (int q = 0; q < w; ++q) carry += sm.chunk[q][lane];
+    if (w == 7) {
+        sm.total[lane] = carry + sum;
+        if (lane == 0) s_cprefix[th] = carry + sum;
+    }
+#pragma unroll 4
+    for (int band = b0; band < b1; ++band) {
+        const uint32_t n = s_table[band * kAreaBins + lane];
+        s_table[band * kAreaBins + lane] = static_cast<uint16_t>(min(carry, 0xffffu));
+        if (lane == 0) s_cprefix[band] = carry;
+        carry += n;
+    }
+    __syncthreads();
     if (tid < 32) {
-        // Exclusive scan of the 64 bin totals: lane l holds bins 2l, 2l + 1.
-        const uint32_t t0 = s_total[2 * lane], t1 = s_total[2 * lane + 1];
-        uint32_t incl = t0 + t1;
+        // Exclusive scan of the bin totals (column 0 is no bin).
+        const uint32_t t = lane == 0 ? 0u : sm.total[lane];
+        uint32_t incl = t;
+#pragma unroll
         for (int off = 1; off < 32; off <<= 1) {
             const uint32_t n = __shfl_up_sync(kFull, incl, off);
             if (lane >= off) incl += n;
         }
-        const uint32_t before = incl - t0 - t1;
-        s_base[2 * lane] = before;
-        s_base[2 * lane + 1] = before + t0;
-        st->bin_base[2 * lane] = before;
-        st->bin_base[2 * lane + 1] = before + t0;
+        sm.base[lane] = incl - t;
+        st->bin_base[lane] = 0;
+        st->bin_base[32 + lane] = incl - t;
         if (lane == 31) {
             st->counts[0] = incl;
             sm.limit = min(incl, static_cast<uint32_t>(d.max_candidates));
@@ -888,38 +891,16 @@ __device__ __forceinline__ bool stage_cand(const BatchDesc* __restrict__ b, int 
             sm.nsmall = 0;
         }
     }
-
+    __syncthreads();
     // Placement (reference k_order_candidates :642-654): candidate j of the
     // frame, flattened over the bands' lists, goes to bin base + earlier
-    // bands' count in its bin + its rank in the band.  Block scan of the
-    // per-band list lengths first.
-    const int chunk = (th + blockDim.x - 1) / blockDim.x;
-    const int cb0 = min(th, tid * chunk), cb1 = min(th, cb0 + chunk);
-    uint32_t own = 0;
-    for (int band = cb0; band < cb1; ++band) own += __ldcg(&d.lroot_count[band]);
-    uint32_t incl = own;
-    for (int off = 1; off < 32; off <<= 1) {
-        const uint32_t v = __shfl_up_sync(kFull, incl, off);
-        if (lane >= off) incl += v;
-    }
-    if (lane == 31) s_warp_sum[w] = incl;
-    __syncthreads();
-    uint32_t before = incl - own;
-    for (int w2 = 0; w2 < w; ++w2) before += s_warp_sum[w2];
-    for (int band = cb0; band < cb1; ++band) {
-        s_cprefix[band] = before;
-        before += __ldcg(&d.lroot_count[band]);
-    }
-    if (tid == blockDim.x - 1) s_cprefix[th] = before;
-    __syncthreads();
+    // bands' count in its bin + its rank in the band.  Four candidates per thread and
+    // pass, their loads in flight together.
     const uint32_t all = s_cprefix[th];
     const uint32_t limit = sm.limit;
-    // Four candidates per thread and pass, their loads in flight together:
-    // slot and bin word (one position of both band lists), then the band's
-    // bin prefix.
     constexpr int kUnroll = 4;
     for (uint32_t j0 = tid; j0 < all; j0 += kUnroll * blockDim.x) {
-        uint32_t slot[kUnroll], meta[kUnroll], prev[kUnroll];
+        uint32_t slot[kUnroll], meta[kUnroll];
         int band[kUnroll];
 #pragma unroll
         for (int u = 0; u < kUnroll; ++u) {
@@ -939,12 +920,9 @@ __device__ __forceinline__ bool stage_cand(const BatchDesc* __restrict__ b, int 
         }
 #pragma unroll
         for (int u = 0; u < kUnroll; ++u) {
-            if (band[u] >= 0) prev[u] = __ldcg(&d.band_bins[band[u] * 64 + (meta[u] >> 24)]);
-        }
-#pragma unroll
-        for (int u = 0; u < kUnroll; ++u) {
             if (band[u] < 0) continue;
-            const uint32_t pos = s_base[meta[u] >> 24] + prev[u] + (meta[u] & 0x7fffffu);
+            const uint32_t bin = (meta[u] >> 24) - 32u;
+            const uint32_t pos = sm.base[bin] + s_table[band[u] * kAreaBins + bin] + (meta[u] & 0x7fffffu);
             if (pos < limit) {
                 d.candidates[pos] = slot[u];
                 // The fit/decode work lists, split by size once here: big

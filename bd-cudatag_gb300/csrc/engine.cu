@@ -295,7 +295,7 @@ Plan* Plan::create(const std::vector<PlanFrame>& frames, const PlanConfig& confi
     std::memset(&hd, 0, sizeof(hd));
     hd.frames = nf;
     std::vector<size_t> off_frame(nf), off_tmin(nf), off_tmax(nf), off_lo(nf), off_hi(nf),
-        off_bits(nf), off_rc(nf), off_runs(nf), off_parent(nf), off_area(nf), off_bbox(nf),
+        off_bits(nf), off_rc(nf), off_wf(nf), off_runs(nf), off_parent(nf), off_area(nf), off_bbox(nf),
         off_meta(nf), off_bands(nf), off_cands(nf), off_hull(nf), off_quads(nf), off_dec(nf),
         off_lroots(nf), off_lcount(nf), off_mode(nf), off_fit(nf);
     im.frame_offset.resize(nf);
@@ -352,6 +352,7 @@ Plan* Plan::create(const std::vector<PlanFrame>& frames, const PlanConfig& confi
         off_hi[i] = carve.take(sizeof(int32_t) * d.tile_h);
         off_bits[i] = carve.take(sizeof(uint32_t) * d.words * f.height);
         off_rc[i] = carve.take(sizeof(uint32_t) * f.height);
+        off_wf[i] = carve.take(sizeof(uint16_t) * d.words * f.height);
         off_runs[i] = carve.take(sizeof(uint32_t) * slots);
         off_parent[i] = carve.take(sizeof(uint32_t) * slots);
         off_area[i] = carve.take(sizeof(uint32_t) * slots);
@@ -393,6 +394,7 @@ Plan* Plan::create(const std::vector<PlanFrame>& frames, const PlanConfig& confi
         d.row_hi = reinterpret_cast<int32_t*>(base + off_hi[i]);
         d.bits = reinterpret_cast<uint32_t*>(base + off_bits[i]);
         d.row_count = reinterpret_cast<uint32_t*>(base + off_rc[i]);
+        d.word_first = reinterpret_cast<uint16_t*>(base + off_wf[i]);
         d.runs = reinterpret_cast<uint32_t*>(base + off_runs[i]);
         d.parent = reinterpret_cast<uint32_t*>(base + off_parent[i]);
         d.area = reinterpret_cast<uint32_t*>(base + off_area[i]);

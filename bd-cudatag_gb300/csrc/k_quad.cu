@@ -26,14 +26,9 @@ __global__ void __launch_bounds__(256) k_fit_decode(const BatchDesc* __restrict_
         const int fam = tid >> 3, c = tid & 7;
         s_uv[fam][c] = (c + 0.5f) / static_cast<float>(family_dim(fam));
     }
-    if (tid == 0) {
-        int run = 0;
-        for (int f = 0; f < b->frames; ++f) {
-            s_prefix[f] = run;
-            run += static_cast<int>(b->f[f].state->n_small) * __popc(b->f[f].families & 3u);
-        }
-        s_prefix[b->frames] = run;
-    }
+    frame_prefix(b->frames, s_prefix, [&](int f) {
+        return static_cast<int>(b->f[f].state->n_small) * __popc(b->f[f].families & 3u);
+    });
     __syncthreads();
     QuadSmem& sm = reinterpret_cast<QuadSmem*>(s_dyn)[warp];
     const int total = s_prefix[b->frames];
@@ -66,14 +61,7 @@ __global__ void __launch_bounds__(256, 3) k_fit_decode_big(const BatchDesc* __re
         const int fam = tid >> 3, c = tid & 7;
         s_uv[fam][c] = (c + 0.5f) / static_cast<float>(family_dim(fam));
     }
-    if (tid == 0) {
-        int run = 0;
-        for (int f = 0; f < b->frames; ++f) {
-            s_prefix[f] = run;
-            run += static_cast<int>(b->f[f].state->n_big);
-        }
-        s_prefix[b->frames] = run;
-    }
+    frame_prefix(b->frames, s_prefix, [&](int f) { return static_cast<int>(b->f[f].state->n_big); });
     __syncthreads();
     const int total = s_prefix[b->frames];
     float ux, uy;
@@ -109,17 +97,10 @@ __global__ void __launch_bounds__(256, 3) k_fit_decode_all(const BatchDesc* __re
         const int fam = tid >> 3, c = tid & 7;
         s_uv[fam][c] = (c + 0.5f) / static_cast<float>(family_dim(fam));
     }
-    if (tid == 0) {
-        int big = 0, small = 0;
-        for (int f = 0; f < b->frames; ++f) {
-            s_big[f] = big;
-            s_small[f] = small;
-            big += static_cast<int>(b->f[f].state->n_big);
-            small += static_cast<int>(b->f[f].state->n_small) * __popc(b->f[f].families & 3u);
-        }
-        s_big[b->frames] = big;
-        s_small[b->frames] = small;
-    }
+    frame_prefix(b->frames, s_big, [&](int f) { return static_cast<int>(b->f[f].state->n_big); });
+    frame_prefix(b->frames, s_small, [&](int f) {
+        return static_cast<int>(b->f[f].state->n_small) * __popc(b->f[f].families & 3u);
+    });
     __syncthreads();
     float ux, uy;
     {

@@ -124,6 +124,8 @@ struct FrameDesc {
     int32_t* row_hi;
     uint32_t* bits;                // height * words, 1 = white
     uint32_t* row_count;           // height
+    uint16_t* word_first;          // height * words: runs of the row before each word (rows of the
+                                   // ROI bands)
     uint32_t* runs;                // slots (height * row_cap): x0 | x1 << 16
     uint32_t* parent;              // slots: union-find, then the root of every run
     uint32_t* area;                // slots (valid at roots)

@@ -357,6 +357,7 @@ __device__ __forceinline__ void stage_binarize(const BatchDesc* __restrict__ b, 
         uint32_t index = first_index;
         for (int c = c0; c < c1; ++c) {
             const uint32_t m = sm_bits[w * bits_words + c];
+            d.word_first[static_cast<int64_t>(y) * words + c] = static_cast<uint16_t>(index);
             uint32_t starts = ~m & ((m << 1) | 1u);
             const int last = min(31, W - 1 - (c << 5));
             while (starts) {

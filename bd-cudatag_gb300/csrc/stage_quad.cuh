@@ -27,117 +27,111 @@ __device__ __forceinline__ uint32_t pack_point(int x, int y) {
 }
 
 // hull_to_quad (reference :736-831) run by one warp: lane i holds hull
-// vertex i; each round drops the vertex whose triangle with its neighbours
-// has the smallest area (first index on ties, as the reference's strict <),
-// found with a warp arg-min instead of a serial scan.  The remaining checks
-// run on lane 0 with the reference's expressions.  Returns the result in all
-// lanes.
-__device__ bool hull_to_quad_warp(const uint32_t* hull, int count, float quad[4][2], int lane) {
+// vertex i (packed) and both neighbours' coordinates; each round drops the vertex whose
+// triangle with its neighbours has the smallest area (first index on ties, as
+// the reference's strict <), found with a warp arg-min instead of a serial
+// scan.  The vertices form a ring of links, so only the two neighbours of the
+// dropped one take new coordinates and a new area.  The remaining
+// checks run on lanes 0-3, one corner each, with the reference's expressions;
+// sums are formed in its order.  Returns the verdict in all lanes and
+// corner i in lane i of *cx, *cy (i < 4).
+__device__ bool hull_to_quad_warp(uint32_t vertex, int count, float* cx_out, float* cy_out, int lane) {
     if (count < 4 || count > kMaxHullVertices || count > 32) return false;
-    float vx = lane < count ? static_cast<float>(hull[lane] & 0xffffu) : 0.0f;
-    float vy = lane < count ? static_cast<float>(hull[lane] >> 16) : 0.0f;
+    const float vx = static_cast<float>(vertex & 0xffffu);
+    const float vy = static_cast<float>(vertex >> 16);
+    int prev = lane == 0 ? count - 1 : lane - 1;
+    int next = lane + 1 >= count ? 0 : lane + 1;
+    float pvx = __shfl_sync(kFull, vx, prev & 31), pvy = __shfl_sync(kFull, vy, prev & 31);
+    float nvx = __shfl_sync(kFull, vx, next & 31), nvy = __shfl_sync(kFull, vy, next & 31);
+    bool alive = lane < count;
     while (count > 4) {
-        // Cyclic neighbours (lanes >= count compute garbage that is unused).
-        const int prev = lane == 0 ? count - 1 : lane - 1;
-        const int next = lane + 1 >= count ? 0 : lane + 1;
-        const float pvx = __shfl_sync(kFull, vx, prev), pvy = __shfl_sync(kFull, vy, prev);
-        const float nvx = __shfl_sync(kFull, vx, next), nvy = __shfl_sync(kFull, vy, next);
-        float area = FLT_MAX;
-        if (lane < count) {
+        uint32_t key = 0xffffffffu;
+        if (alive) {
             const float ax = vx - pvx;
             const float ay = vy - pvy;
             const float bx = nvx - vx;
             const float by = nvy - vy;
-            area = fabsf(ax * by - ay * bx) * 0.5f;
+            float area = fabsf(ax * by - ay * bx) * 0.5f;
             if (!(area < FLT_MAX)) area = FLT_MAX;
+            key = __float_as_uint(area);  // areas are >= 0: their bits order like the values
         }
-        // Areas are >= 0, so their bit patterns order like the values.
-        const uint32_t key = __float_as_uint(area);
         const uint32_t best_key = __reduce_min_sync(kFull, key);
-        if (best_key == __float_as_uint(FLT_MAX)) return false;
-        const int idx = __ffs(__ballot_sync(kFull, lane < count && key == best_key)) - 1;
-        const float sx = __shfl_down_sync(kFull, vx, 1), sy = __shfl_down_sync(kFull, vy, 1);
-        if (lane >= idx) {
-            vx = sx;
-            vy = sy;
+        if (best_key >= __float_as_uint(FLT_MAX)) return false;
+        const int idx = __ffs(__ballot_sync(kFull, key == best_key)) - 1;
+        const int links = __shfl_sync(kFull, prev | (next << 8), idx);
+        const float ipx = __shfl_sync(kFull, pvx, idx), ipy = __shfl_sync(kFull, pvy, idx);
+        const float inx = __shfl_sync(kFull, nvx, idx), iny = __shfl_sync(kFull, nvy, idx);
+        const int p = links & 0xff, n = links >> 8;
+        if (lane == idx) alive = false;
+        if (lane == p) {
+            next = n;
+            nvx = inx;
+            nvy = iny;
+        }
+        if (lane == n) {
+            prev = p;
+            pvx = ipx;
+            pvy = ipy;
         }
         --count;
     }
-    float qx[4], qy[4];
+    // The four left, in order, in every lane.
+    uint32_t left = __ballot_sync(kFull, alive);
+    float x[4], y[4];
+#pragma unroll
     for (int i = 0; i < 4; ++i) {
-        qx[i] = __shfl_sync(kFull, vx, i);
-        qy[i] = __shfl_sync(kFull, vy, i);
+        const int at = __ffs(left) - 1;
+        left &= left - 1u;
+        x[i] = __shfl_sync(kFull, vx, at);
+        y[i] = __shfl_sync(kFull, vy, at);
     }
-    int ok = 0;
-    if (lane == 0) {
-        float* x = qx;
-        float* y = qy;
-        ok = 1;
-        float area2 = 0.0f;
-        for (int i = 0; i < 4; ++i) {
-            const int j = (i + 1) & 3;
-            area2 += x[i] * y[j] - x[j] * y[i];
-        }
-        if (fabsf(area2) < 24.0f) ok = 0;
-        if (ok && area2 < 0.0f) {
-            for (int i = 0; i < 2; ++i) {
-                const float tx = x[i + 1], tyy = y[i + 1];
-                x[i + 1] = x[3 - i];
-                y[i + 1] = y[3 - i];
-                x[3 - i] = tx;
-                y[3 - i] = tyy;
-            }
-        }
-        float min_side = FLT_MAX, max_side = 0.0f;
-        for (int i = 0; ok && i < 4; ++i) {
-            const int j = (i + 1) & 3;
-            const float ex = x[j] - x[i];
-            const float ey = y[j] - y[i];
-            const float len = sqrtf(ex * ex + ey * ey);
-            if (len < 4.0f) {
-                ok = 0;
-                break;
-            }
-            min_side = fminf(min_side, len);
-            max_side = fmaxf(max_side, len);
-            const int p = (i + 3) & 3;
-            const float ax = x[i] - x[p];
-            const float ay = y[i] - y[p];
-            const float bx = x[j] - x[i];
-            const float by = y[j] - y[i];
-            if (ax * by - ay * bx <= 0.0f) {
-                ok = 0;
-                break;
-            }
-            const float dot = ax * bx + ay * by;
-            const float n1 = sqrtf(ax * ax + ay * ay);
-            const float n2 = sqrtf(bx * bx + by * by);
-            if (n1 < 1e-3f || n2 < 1e-3f || fabsf(dot / (n1 * n2)) > 0.97f) {
-                ok = 0;
-                break;
-            }
-        }
-        if (ok && max_side > 12.0f * min_side) ok = 0;
-        if (ok) {
-            const float cx = 0.25f * (x[0] + x[1] + x[2] + x[3]);
-            const float cy = 0.25f * (y[0] + y[1] + y[2] + y[3]);
-            for (int i = 0; i < 4; ++i) {
-                const float dx = x[i] - cx;
-                const float dy = y[i] - cy;
-                const float len = sqrtf(dx * dx + dy * dy);
-                if (len > 1e-3f) {
-                    x[i] += dx / len * 0.65f;
-                    y[i] += dy / len * 0.65f;
-                }
-            }
-        }
-    }
-    ok = __shfl_sync(kFull, ok, 0);
+    float area2 = 0.0f;
+#pragma unroll
     for (int i = 0; i < 4; ++i) {
-        quad[i][0] = __shfl_sync(kFull, qx[i], 0);
-        quad[i][1] = __shfl_sync(kFull, qy[i], 0);
+        const int j = (i + 1) & 3;
+        area2 += x[i] * y[j] - x[j] * y[i];
     }
-    return ok != 0;
+    if (fabsf(area2) < 24.0f) return false;
+    if (area2 < 0.0f) {  // the other way round: corners 1 and 3 change places
+        float t = x[1];
+        x[1] = x[3];
+        x[3] = t;
+        t = y[1];
+        y[1] = y[3];
+        y[3] = t;
+    }
+    // Corner i on lane i, with the side to corner i + 1; a: the side from
+    // corner i - 1, b: its own.
+    const int i = lane & 3;
+    const float cx = i == 0 ? x[0] : (i == 1 ? x[1] : (i == 2 ? x[2] : x[3]));
+    const float cy = i == 0 ? y[0] : (i == 1 ? y[1] : (i == 2 ? y[2] : y[3]));
+    const int jl = (lane + 1) & 3, pl = (lane + 3) & 3;
+    const float bx = __shfl_sync(kFull, cx, jl) - cx;
+    const float by = __shfl_sync(kFull, cy, jl) - cy;
+    const float len = sqrtf(bx * bx + by * by);
+    const float ax = __shfl_sync(kFull, bx, pl), ay = __shfl_sync(kFull, by, pl);
+    const float n1 = __shfl_sync(kFull, len, pl);
+    bool bad = len < 4.0f;
+    bad = bad || ax * by - ay * bx <= 0.0f;
+    const float dot = ax * bx + ay * by;
+    bad = bad || n1 < 1e-3f || len < 1e-3f || fabsf(dot / (n1 * len)) > 0.97f;
+    const uint32_t bad_lanes = __ballot_sync(kFull, bad);
+    if (bad_lanes & 0xfu) return false;
+    float min_side = len, max_side = len;
+#pragma unroll
+    for (int off = 1; off < 4; off <<= 1) {
+        min_side = fminf(min_side, __shfl_xor_sync(kFull, min_side, off));
+        max_side = fmaxf(max_side, __shfl_xor_sync(kFull, max_side, off));
+    }
+    if (max_side > 12.0f * min_side) return false;
+    const float mx = 0.25f * (x[0] + x[1] + x[2] + x[3]);
+    const float my = 0.25f * (y[0] + y[1] + y[2] + y[3]);
+    const float dx = cx - mx;
+    const float dy = cy - my;
+    const float out = sqrtf(dx * dx + dy * dy);
+    *cx_out = out > 1e-3f ? cx + dx / out * 0.65f : cx;
+    *cy_out = out > 1e-3f ? cy + dy / out * 0.65f : cy;
+    return true;
 }
 
 __device__ __forceinline__ bool intersect_lines(const float li[4], const float lj[4], float* x,
@@ -737,9 +731,13 @@ __device__ int decode_rotations_warp(const uint8_t* __restrict__ gray, const Fra
 
 // Per-warp shared memory of k_fit_decode.
 struct QuadSmem {
-    // The probe profiles live only while edges are refined, the decode
-    // cells only while the quad is decoded: they share the space.
+    // The boundary rows live only while the hull is built, the probe profiles
+    // only while edges are refined, the decode cells only while the quad is
+    // decoded: they share the space.
     union {
+        struct {
+            float lx[32], rx[32], y[32];
+        } rows;
         float mags[32 * kMaxProbes];  // one probe profile per lane
         struct {
             float raw[4][64];         // per rotation: samples, then differences
@@ -755,69 +753,123 @@ struct QuadSmem {
 };
 
 // Leftmost / rightmost run of component `root` in row y within [x0, x1]
-// (reference collect_row_extremes :676-715): binary search for the first
-// run ending at or after x0, then runs in order until one starts past x1.
+// (reference collect_row_extremes :676-715).  The runs between the two columns
+// follow from the row's bits and the run counts before its words, without
+// a search, and they are looked through from both ends until a run of the
+// component turns up: two dependent rounds of loads in most rows, where a
+// search and a walk over every run took ten.  Returns the left and
+// right ends, or -1 twice.
 __device__ __forceinline__ void row_extremes(const FrameDesc& d, uint32_t root, int x0, int x1, int y,
-                                             uint32_t* left_point, uint32_t* right_point) {
-    const int n = static_cast<int>(d.row_count[y]);
+                                             int* left_out, int* right_out) {
+    const int64_t row_words = static_cast<int64_t>(y) * d.words;
+    const int w0 = x0 >> 5, w1 = x1 >> 5;
+    const uint32_t m0 = d.bits[row_words + w0], m1 = d.bits[row_words + w1];
+    const int f0 = d.word_first[row_words + w0], f1 = d.word_first[row_words + w1];
+    const uint32_t ends = ~m0 & ((m0 >> 1) | 0x80000000u);  // last pixels of the word's runs
+    const uint32_t starts = ~m1 & ((m1 << 1) | 1u);
+    const int first = f0 + __popc(ends & ((1u << (x0 & 31)) - 1u));
+    const int last = f1 + __popc(starts & (kFull >> (31 - (x1 & 31)))) - 1;
     const uint32_t* row_runs = d.runs + static_cast<int64_t>(y) * d.row_cap;
     const uint32_t* row_label = d.parent + static_cast<int64_t>(y) * d.row_cap;
-    // First run ending at or after x0 (runs of a row are sorted): eight-way
-    // steps of seven independent loads, then the last <= 8 runs at once.
-    int lo = 0, hi = n;  // the answer lies in [lo, hi]; hi = n: none
-    while (hi - lo > 8) {
-        const int span = hi - lo;
-        uint32_t v[7];
-#pragma unroll
-        for (int k = 0; k < 7; ++k) v[k] = row_runs[lo + (span * (k + 1)) / 8];
-        int nlo = lo, nhi = hi;
-#pragma unroll
-        for (int k = 6; k >= 0; --k) {
-            const int idx = lo + (span * (k + 1)) / 8;
-            if (static_cast<int>(v[k] >> 16) >= x0) nhi = idx; else if (nlo == lo) nlo = idx + 1;
-        }
-        lo = nlo;
-        hi = nhi;
-    }
-    int first = hi;
-    {
-        uint32_t v[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) v[k] = row_runs[min(lo + k, max(n - 1, 0))];
-#pragma unroll
-        for (int k = 7; k >= 0; --k) {
-            if (lo + k < hi && static_cast<int>(v[k] >> 16) >= x0) first = lo + k;
-        }
-    }
     int left = -1, right = -1;
-    // Runs two at a time (no padding loads past the end of the row).
-    for (int k = first; k < n; k += 2) {
-        uint32_t rr[2] = {}, lab[2] = {};
+    constexpr int kStep = 4;
+    for (int a = first, b = last; a <= last && (left < 0 || right < 0); a += kStep, b -= kStep) {
+        uint32_t la[kStep], lb[kStep], ra[kStep], rb[kStep];
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            if (k + j < n) {
-                rr[j] = row_runs[k + j];
-                lab[j] = row_label[k + j];
+        for (int k = 0; k < kStep; ++k) {
+            const int ia = min(a + k, last), ib = max(b - k, first);
+            la[k] = row_label[ia];
+            lb[k] = row_label[ib];
+            ra[k] = row_runs[ia];
+            rb[k] = row_runs[ib];
+        }
+        if (left < 0) {
+#pragma unroll
+            for (int k = kStep - 1; k >= 0; --k) {
+                if (la[k] == root) left = static_cast<int>(ra[k] & 0xffffu);
             }
         }
-        bool stop = false;
+        if (right < 0) {
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            if (stop || k + j >= n) continue;
-            const int rx0 = static_cast<int>(rr[j] & 0xffffu);
-            const int rx1 = static_cast<int>(rr[j] >> 16);
-            if (rx0 > x1) {
-                stop = true;
-                continue;
+            for (int k = kStep - 1; k >= 0; --k) {
+                if (lb[k] == root) right = static_cast<int>(rb[k] >> 16);
             }
-            if (lab[j] != root) continue;
-            left = left < 0 ? rx0 : min(left, rx0);
-            right = right < 0 ? rx1 : max(right, rx1);
         }
-        if (stop) break;
     }
-    *left_point = left < 0 ? kNone : pack_point(left, y);
-    *right_point = right < 0 ? kNone : pack_point(right, y);
+    *left_out = left;
+    *right_out = right;
+}
+
+// Best boundary point of this lane's probe direction (ux, uy) over rows
+// [begin, end) of a boundary in shared memory: the first point of largest
+// projection, rows in order, left before right (reference :1134-1170).
+// Both ends of a row share y, so the row costs three products; a row
+// without a point holds NaN, whose projection never wins.
+__device__ __forceinline__ void probe_rows(const float* lx, const float* rx, const float* py, int begin,
+                                           int end, float ux, float uy, float* best_dot, int* pick) {
+    float best = *best_dot;
+    int at = *pick;
+#pragma unroll 4
+    for (int s = begin; s < end; ++s) {
+        const float yy = py[s] * uy;
+        const float dl = lx[s] * ux + yy;
+        const float dr = rx[s] * ux + yy;
+        if (dl > best) {
+            best = dl;
+            at = 2 * s;
+        }
+        if (dr > best) {
+            best = dr;
+            at = 2 * s + 1;
+        }
+    }
+    *best_dot = best;
+    *pick = at;
+}
+
+// One warp: the hull from every direction's best point (lane = direction;
+// kNone: none) and its quad.  Hull: extremes in direction order without repeats
+// of the previous kept point, and without a last point equal to the first.  The
+// previous kept point equals the nearest earlier valid extreme.  Returns whether
+// there is a quad, in all lanes, and coordinate l of its corners in lane l of
+// *coordinate (l < 8).
+__device__ __forceinline__ bool hull_quad_warp(uint32_t point, int lane, uint32_t* s_hull, float* coordinate) {
+    const bool valid = point != kNone;
+    const uint32_t vmask = __ballot_sync(kFull, valid);
+    const uint32_t earlier = vmask & lanemask_lt();
+    const int prev_lane = earlier ? 31 - __clz(earlier) : 0;
+    const uint32_t prev_point = __shfl_sync(kFull, point, prev_lane);
+    const bool keep = valid && (earlier == 0 || prev_point != point);
+    const uint32_t kmask = __ballot_sync(kFull, keep);
+    if (keep) s_hull[__popc(kmask & lanemask_lt())] = point;
+    __syncwarp();
+    int hc = __popc(kmask);
+    const uint32_t vertex = lane < hc ? s_hull[lane] : 0u;
+    // Trailing vertices equal to the first are dropped.
+    const uint32_t differs = __ballot_sync(kFull, lane < hc && vertex != s_hull[0]);
+    hc = hc > 0 ? 32 - __clz(differs | 1u) : 0;
+    float cx = 0.0f, cy = 0.0f;
+    const bool ok = hull_to_quad_warp(vertex, hc, &cx, &cy, lane);
+    const float x = __shfl_sync(kFull, cx, lane >> 1), y = __shfl_sync(kFull, cy, lane >> 1);
+    *coordinate = (lane & 1) ? y : x;
+    return ok;
+}
+
+__device__ __forceinline__ uint32_t picked_point(const float* lx, const float* rx, const float* py, int pick) {
+    if (pick < 0) return kNone;
+    const int s = pick >> 1;
+    return pack_point(static_cast<int>((pick & 1) ? rx[s] : lx[s]), static_cast<int>(py[s]));
+}
+
+__device__ __forceinline__ void boundary_row(const FrameDesc& d, uint32_t root, uint4 bb, int rows, int kept,
+                                             int s, float* lx, float* rx, float* py) {
+    const int y0 = static_cast<int>(bb.y);
+    const int y = y0 + (kept == rows ? s : (s * (rows - 1)) / (kept - 1));  // kept < rows: kept > 1
+    int left, right;
+    row_extremes(d, root, static_cast<int>(bb.x), static_cast<int>(bb.z), y, &left, &right);
+    *lx = left < 0 ? bdmath::quiet_nan() : static_cast<float>(left);
+    *rx = right < 0 ? bdmath::quiet_nan() : static_cast<float>(right);
+    *py = static_cast<float>(y);
 }
 
 // Refinement and decode of one (candidate, family) item by one warp, from
@@ -896,79 +948,29 @@ __device__ __forceinline__ void fit_small_item(const BatchDesc* __restrict__ b,
     const int64_t stride = io[fi].stride;
     const uint32_t root = d.candidates[ci];
     const uint4 bb = reinterpret_cast<const uint4*>(d.bbox)[root];
-    const int x0 = static_cast<int>(bb.x), y0 = static_cast<int>(bb.y);
-    const int x1 = static_cast<int>(bb.z), y1 = static_cast<int>(bb.w);
-    const int rows = y1 - y0 + 1;
+    const int rows = static_cast<int>(bb.w - bb.y) + 1;
     const int kept = min(rows, kMaxBoundaryRows);
 
-    // Boundary points in reference order (row s: left, then right) go
-    // to every lane by shuffles; lane = direction keeps the first point
-    // of largest projection.  The points travel as float coordinates,
-    // converted once by the lane that found them (NaN for a row without a
-    // point: its projection never wins), and the winning point's packed
-    // form is fetched once per round.
+    // Boundary points, lane = row, then lane = direction.
     float best_dot = -FLT_MAX;
     uint32_t best_point = kNone;
-    const float none = bdmath::quiet_nan();
     for (int s0 = 0; s0 < kept; s0 += 32) {
-        uint32_t lp = kNone, rp = kNone;
         const int s = s0 + lane;
         if (s < kept) {
-            const int y = y0 + (kept == rows ? s : (s * (rows - 1)) / (kept - 1));  // kept < rows: kept > 1
-            row_extremes(d, root, x0, x1, y, &lp, &rp);
+            boundary_row(d, root, bb, rows, kept, s, &sm.rows.lx[lane], &sm.rows.rx[lane], &sm.rows.y[lane]);
         }
-        const float lx = lp != kNone ? static_cast<float>(lp & 0xffffu) : none;
-        const float ly = lp != kNone ? static_cast<float>(lp >> 16) : none;
-        const float rx = rp != kNone ? static_cast<float>(rp & 0xffffu) : none;
-        const float ry = rp != kNone ? static_cast<float>(rp >> 16) : none;
-        const int count = min(32, kept - s0);
-        int pick = -1;  // 2 * row + side of this round's best point
-        for (int k = 0; k < count; ++k) {
-            const float ax = __shfl_sync(kFull, lx, k), ay = __shfl_sync(kFull, ly, k);
-            const float bx = __shfl_sync(kFull, rx, k), by = __shfl_sync(kFull, ry, k);
-            const float dl = ax * ux + ay * uy;
-            if (dl > best_dot) {
-                best_dot = dl;
-                pick = 2 * k;
-            }
-            const float dr = bx * ux + by * uy;
-            if (dr > best_dot) {
-                best_dot = dr;
-                pick = 2 * k + 1;
-            }
-        }
-        const uint32_t cl = __shfl_sync(kFull, lp, max(pick, 0) >> 1);
-        const uint32_t cr = __shfl_sync(kFull, rp, max(pick, 0) >> 1);
-        if (pick >= 0) best_point = (pick & 1) ? cr : cl;
+        __syncwarp();
+        int pick = -1;
+        probe_rows(sm.rows.lx, sm.rows.rx, sm.rows.y, 0, min(32, kept - s0), ux, uy, &best_dot, &pick);
+        if (pick >= 0) best_point = picked_point(sm.rows.lx, sm.rows.rx, sm.rows.y, pick);
+        __syncwarp();
     }
-    // Hull: extremes in direction order without repeats of the previous
-    // kept point, and without a last point equal to the first.  The
-    // previous kept point equals the nearest earlier valid extreme.
-    const bool valid = best_point != kNone;
-    const uint32_t vmask = __ballot_sync(kFull, valid);
-    const uint32_t earlier = vmask & lanemask_lt();
-    const int prev_lane = earlier ? 31 - __clz(earlier) : 0;
-    const uint32_t prev_point = __shfl_sync(kFull, best_point, prev_lane);
-    const bool keep = valid && (earlier == 0 || prev_point != best_point);
-    const uint32_t kmask = __ballot_sync(kFull, keep);
-    if (keep) sm.hull[__popc(kmask & lanemask_lt())] = best_point;
-    __syncwarp();
-    int hc = __popc(kmask);
-    while (hc > 1 && sm.hull[0] == sm.hull[hc - 1]) --hc;
-
-    float quad[4][2] = {};
-    const bool quad_ok = hull_to_quad_warp(sm.hull, hc, quad, lane);
-    {
-        float v = 0.0f;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) v = lane == k ? quad[k >> 1][k & 1] : v;
-        if (lane < 8) {
-            sm.hq[lane >> 1][lane & 1] = v;
-            sm.q[lane >> 1][lane & 1] = v;
-            if (first_family) {
-                d.hull_quads[static_cast<int64_t>(ci) * 8 + lane] = quad_ok ? v : bdmath::quiet_nan();
-            }
-        }
+    float v;
+    const bool quad_ok = hull_quad_warp(best_point, lane, sm.hull, &v);
+    if (lane < 8) {
+        sm.hq[lane >> 1][lane & 1] = v;
+        sm.q[lane >> 1][lane & 1] = v;
+        if (first_family) d.hull_quads[static_cast<int64_t>(ci) * 8 + lane] = quad_ok ? v : bdmath::quiet_nan();
     }
     if (lane == 0 && quad_ok && first_family) atomicAdd(&d.state->counts[3], 1u);
     __syncwarp();
@@ -977,9 +979,8 @@ __device__ __forceinline__ void fit_small_item(const BatchDesc* __restrict__ b,
 
 // Shared memory of fit_big_item.
 struct BigSmem {
-    uint32_t boundary[2 * kMaxBoundaryRows];
     float probe_dot[8][kFitDirections];
-    uint32_t probe_point[8][kFitDirections];
+    int probe_pick[8][kFitDirections];
     uint32_t s_hull[kFitDirections];
     float hull_quad[4][2];
     float fit_quad[2][4][2];
@@ -987,7 +988,12 @@ struct BigSmem {
     int edge_have[2][4];
     int quad_ok;
     int s_done[2];
-    float s_mags[8][16 * kMaxProbes];
+    union {  // the boundary is done when the edges are probed
+        struct {
+            float lx[kMaxBoundaryRows], rx[kMaxBoundaryRows], y[kMaxBoundaryRows];
+        } rows;
+        float s_mags[8][16 * kMaxProbes];
+    };
     float s_raw[4][4][64];
     float s_sharp[4][4][64];
     VariantResult s_res[4];
@@ -1014,64 +1020,34 @@ __device__ __forceinline__ void fit_big_item(const BatchDesc* __restrict__ b,
     const int64_t stride = io[fi].stride;
     const uint32_t root = d.candidates[ci];
     const uint4 bb = reinterpret_cast<const uint4*>(d.bbox)[root];
-    const int x0 = static_cast<int>(bb.x), y0 = static_cast<int>(bb.y);
-    const int x1 = static_cast<int>(bb.z), y1 = static_cast<int>(bb.w);
-    const int rows = y1 - y0 + 1;
+    const int rows = static_cast<int>(bb.w - bb.y) + 1;
     const int kept = min(rows, kMaxBoundaryRows);
-    const int points = 2 * kept;
 
     for (int s = tid; s < kept; s += blockDim.x) {
-        const int y = y0 + (kept == rows ? s : (s * (rows - 1)) / (kept - 1));  // kept < rows: kept > 1
-        row_extremes(d, root, x0, x1, y, &sm.boundary[2 * s], &sm.boundary[2 * s + 1]);
+        boundary_row(d, root, bb, rows, kept, s, &sm.rows.lx[s], &sm.rows.rx[s], &sm.rows.y[s]);
     }
     __syncthreads();
     // Extreme point per direction over this warp's slice; slices
     // are merged in order, so the first point still wins ties.
+    float best_dot = -FLT_MAX;
+    int pick = -1;
     {
-        const int slice = (points + kWarps - 1) / kWarps;
-        const int begin = warp * slice;
-        const int end = min(points, begin + slice);
-        float best_dot = -FLT_MAX;
-        uint32_t best_point = kNone;
-        for (int i = begin; i < end; ++i) {
-            const uint32_t p = sm.boundary[i];
-            if (p == kNone) continue;
-            const float dd =
-                static_cast<float>(p & 0xffffu) * ux + static_cast<float>(p >> 16) * uy;
-            if (dd > best_dot) {
-                best_dot = dd;
-                best_point = p;
-            }
-        }
+        const int slice = (kept + kWarps - 1) / kWarps;
+        probe_rows(sm.rows.lx, sm.rows.rx, sm.rows.y, min(kept, warp * slice), min(kept, (warp + 1) * slice), ux, uy,
+                   &best_dot, &pick);
         sm.probe_dot[warp][lane] = best_dot;
-        sm.probe_point[warp][lane] = best_point;
+        sm.probe_pick[warp][lane] = pick;
     }
     __syncthreads();
     if (warp == 0) {
-        float best_dot = -FLT_MAX;
-        uint32_t best_point = kNone;
-        for (int p = 0; p < kWarps; ++p) {
+        for (int p = 1; p < kWarps; ++p) {
             if (sm.probe_dot[p][lane] > best_dot) {
                 best_dot = sm.probe_dot[p][lane];
-                best_point = sm.probe_point[p][lane];
+                pick = sm.probe_pick[p][lane];
             }
         }
-        const bool valid = best_point != kNone;
-        const uint32_t vmask = __ballot_sync(kFull, valid);
-        const uint32_t earlier = vmask & lanemask_lt();
-        const int prev_lane = earlier ? 31 - __clz(earlier) : 0;
-        const uint32_t prev_point = __shfl_sync(kFull, best_point, prev_lane);
-        const bool keep = valid && (earlier == 0 || prev_point != best_point);
-        const uint32_t kmask = __ballot_sync(kFull, keep);
-        if (keep) sm.s_hull[__popc(kmask & lanemask_lt())] = best_point;
-        __syncwarp();
-        int hc = __popc(kmask);
-        while (hc > 1 && sm.s_hull[0] == sm.s_hull[hc - 1]) --hc;
-        float quad[4][2] = {};
-        const bool ok = hull_to_quad_warp(sm.s_hull, hc, quad, lane);
-        float v = 0.0f;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) v = lane == k ? quad[k >> 1][k & 1] : v;
+        float v;
+        const bool ok = hull_quad_warp(picked_point(sm.rows.lx, sm.rows.rx, sm.rows.y, pick), lane, sm.s_hull, &v);
         if (lane < 8) {
             sm.hull_quad[lane >> 1][lane & 1] = v;
             sm.fit_quad[0][lane >> 1][lane & 1] = v;
@@ -1165,6 +1141,29 @@ __device__ __forceinline__ void fit_big_item(const BatchDesc* __restrict__ b,
         }
     }
     __syncthreads();
+}
+
+// Exclusive prefix over the frames of a batch of n(f), into s_prefix[0 ..
+// frames], by warp 0 (lane = frame); the caller synchronises.  A thread that
+// walked the frames would wait for each one's state in turn.
+template <typename Count>
+__device__ __forceinline__ void frame_prefix(int frames, int* s_prefix, const Count& n) {
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x;
+        int carry = 0;
+        for (int f0 = 0; f0 < frames; f0 += 32) {
+            const int own = f0 + lane < frames ? n(f0 + lane) : 0;
+            int incl = own;
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const int v = __shfl_up_sync(kFull, incl, off);
+                if (lane >= off) incl += v;
+            }
+            if (f0 + lane < frames) s_prefix[f0 + lane] = carry + incl - own;
+            carry += __shfl_sync(kFull, incl, 31);
+        }
+        if (lane == 0) s_prefix[frames] = carry;
+    }
 }
 
 }  // namespace

@@ -31,6 +31,17 @@ int prepare_pipeline() {
                              static_cast<int>(fit_all_smem_bytes())) != cudaSuccess) {
         return -1;
     }
+    // Half of an SM's 228 KB as shared memory for both fit kernels: three CTAs of
+    // either, or some of both side by side (an SM takes kernels of one split at a time), and the
+    // rest as L1 for the pixels and runs they gather.  Four 1280x800 frames:
+    // 131 us with half, 139 with the driver's choice, 143 with all, 135 with a
+    // quarter; sixteen such batches in flight: 643, 656, 669 and 774 us.
+    for (const void* kernel : {reinterpret_cast<const void*>(k_fit_decode),
+                               reinterpret_cast<const void*>(k_fit_decode_big)}) {
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 50) != cudaSuccess) {
+            return -1;
+        }
+    }
     int per_sm = 1;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fit_decode_all, 256, fit_all_smem_bytes()) ==
         cudaSuccess) {

@@ -30,6 +30,6 @@ def test_word_edges(left, right, stripes):
 @pytest.mark.parametrize("rows", [1024, 1025, 1300])
 def test_more_rows_than_kept(rows):
     img = np.full((rows + 40, 700), 220, np.uint8)
-    ring(img, 40, 20, 640, 19 + rows, 60)
+    ring(img, 40, 20, 340, 19 + rows, 60)
     img[300:340, 0:20] = 30
     check_frame(img, 0)

@@ -60,6 +60,25 @@ int auto_max_candidates(int width, int height, int configured) {
     return std::min(std::max(next_power_of_two((width * height) / 4096) * 3 / 2, 96), 1024);
 }
 
+// Launch shapes of a new plan.
+//  * Frames up to 2048 px wide label bands in segments of 1024 runs: camera
+//    frames stay below that in nearly every band, and with 28 KB instead of 55
+//    an SM holds six of k_binarize_runs' CTAs, not four (sixteen 4x1280x800
+//    batches in flight 640 -> 617 us, sixteen mixed frames 225 -> 217).  Wider
+//    noisy frames have bands of 5,000 runs, and a segment more costs a union
+//    across it (3840x2160: 139 us with 2048, 150 with 1024).
+//  * k_stats takes two tile rows per CTA when they fit one pass of its threads
+//    and leave a CTA per SM (in flight: 617 -> 605 us); smaller plans keep a CTA
+//    per row.
+LaunchConfig default_launch(const BatchDesc& d, int sm_count) {
+    LaunchConfig lc;
+    int width = 0;
+    for (int f = 0; f < d.frames; ++f) width = std::max(width, d.f[f].width);
+    lc.band_cap = width <= 2048 ? 1024 : 2048;
+    lc.stats_rows = width <= 2048 && d.total_bands >= 2 * sm_count ? 2 : 1;
+    return lc;
+}
+
 struct Plan::Impl {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -370,6 +389,7 @@ Plan* Plan::create(const std::vector<PlanFrame>& frames, const PlanConfig& confi
     }
     hd.band_prefix[nf] = bands;
     hd.total_bands = bands;
+    im.launch_cfg = default_launch(hd, im.sm_count);
     set_stats_rows(hd, im.launch_cfg.stats_rows);
     plan->arena_bytes_ = carve.off;
 

@@ -159,7 +159,8 @@ struct BatchDesc {
     FrameDesc f[kMaxFrames];
 };
 
-// Launch shapes that do not change any result (tuned per plan).
+// Launch shapes that do not change any result (a plan starts from default_launch,
+// engine.cu, and can be tuned).
 constexpr int kMaxQuadWarps = 8;
 struct LaunchConfig {
     int stats_rows = 1;        // tile rows per k_stats CTA: 1, 2 or 4

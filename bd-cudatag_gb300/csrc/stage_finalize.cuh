@@ -10,12 +10,13 @@ namespace bdgb {
 namespace {
 
 struct FinalSmem {
-    DecodeOut in[kMaxDetectionsCap];
-    DecodeOut out[kMaxDetectionsCap];
-    float cx[kMaxDetectionsCap], cy[kMaxDetectionsCap];
+    DecodeOut in[kMaxDetectionsCap];   // compacted detections
+    float cx[kMaxDetectionsCap], cy[kMaxDetectionsCap], limit[kMaxDetectionsCap];
     float h[kMaxDetectionsCap][9];     // homography of each compacted detection
-    int out_in[kMaxDetectionsCap];     // compacted index of each kept detection
-    int rank[kMaxDetectionsCap];       // place of each kept detection, by id
+    // Kept detections: compacted index, id and centre, place by id.
+    int kept_in[kMaxDetectionsCap], kept_id[kMaxDetectionsCap];
+    float kept_cx[kMaxDetectionsCap], kept_cy[kMaxDetectionsCap];
+    int rank[kMaxDetectionsCap];
     uint32_t warp[kFinalThreads / 32];
     int count, kept;
 };
@@ -64,9 +65,6 @@ __device__ void fill_homography(const float corners[8], float H[9]) {
 __device__ __forceinline__ void stage_finalize(const BatchDesc* __restrict__ b, int fi, int fam,
                                                FinalSmem& sm) {
     DecodeOut* s_in = sm.in;
-    DecodeOut* s_out = sm.out;
-    float* s_cx = sm.cx;
-    float* s_cy = sm.cy;
     uint32_t* s_warp = sm.warp;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -113,8 +111,10 @@ __device__ __forceinline__ void stage_finalize(const BatchDesc* __restrict__ b, 
     if (warp > 0) {
         for (int i = tid - 32; i < m; i += kFinalThreads - 32) fill_homography(s_in[i].corners, sm.h[i]);
     } else {
-        int kept = 0;
-        for (int i = 0; i < m; ++i) {
+        // Centre and distance limit of every detection, a lane each; the pass in
+        // arrival order then only compares (it took 400 cycles a detection with
+        // their four square roots in it).
+        for (int i = lane; i < m; i += 32) {
             const DecodeOut& dd = s_in[i];
             float side = 0.0f, cx = 0.0f, cy = 0.0f;
             for (int k = 0; k < 4; ++k) {
@@ -125,34 +125,34 @@ __device__ __forceinline__ void stage_finalize(const BatchDesc* __restrict__ b, 
                 cy += dd.corners[k * 2 + 1];
             }
             side *= 0.25f;
-            cx *= 0.25f;
-            cy *= 0.25f;
-            const float limit = 0.35f * side;
+            sm.cx[i] = cx * 0.25f;
+            sm.cy[i] = cy * 0.25f;
+            sm.limit[i] = 0.35f * side;
+        }
+        __syncwarp();
+        int kept = 0;
+        for (int i = 0; i < m; ++i) {
+            const int id = s_in[i].id;
+            const float cx = sm.cx[i], cy = sm.cy[i], limit = sm.limit[i];
             int duplicate = -1;
             for (int k0 = 0; k0 < kept && duplicate < 0; k0 += 32) {
                 const int k = k0 + lane;
-                const bool hit = k < kept && s_out[k].id == dd.id && fabsf(s_cx[k] - cx) < limit &&
-                                 fabsf(s_cy[k] - cy) < limit;
+                const bool hit = k < kept && sm.kept_id[k] == id && fabsf(sm.kept_cx[k] - cx) < limit &&
+                                 fabsf(sm.kept_cy[k] - cy) < limit;
                 const unsigned bal = __ballot_sync(kFull, hit);
                 if (bal) duplicate = k0 + __ffs(bal) - 1;
             }
+            // kept <= i < m <= maxd: there is room.
+            const int at = duplicate >= 0 ? duplicate : kept;
+            const bool take = duplicate < 0 || s_in[i].margin > s_in[sm.kept_in[duplicate]].margin;
             __syncwarp();
-            if (lane == 0) {
-                if (duplicate >= 0) {
-                    if (dd.margin > s_out[duplicate].margin) {
-                        s_out[duplicate] = dd;
-                        sm.out_in[duplicate] = i;
-                        s_cx[duplicate] = cx;
-                        s_cy[duplicate] = cy;
-                    }
-                } else if (kept < maxd) {
-                    s_out[kept] = dd;
-                    sm.out_in[kept] = i;
-                    s_cx[kept] = cx;
-                    s_cy[kept] = cy;
-                }
+            if (lane == 0 && take) {
+                sm.kept_in[at] = i;
+                sm.kept_id[at] = id;
+                sm.kept_cx[at] = cx;
+                sm.kept_cy[at] = cy;
             }
-            if (duplicate < 0 && kept < maxd) ++kept;
+            if (duplicate < 0) ++kept;
             __syncwarp();
         }
         if (lane == 0) sm.kept = kept;
@@ -161,10 +161,10 @@ __device__ __forceinline__ void stage_finalize(const BatchDesc* __restrict__ b, 
     const int kept = sm.kept;
     bd_detection* dets = result_detections(hdr) + static_cast<int64_t>(fam) * maxd;
     for (int i = tid; i < kept; i += kFinalThreads) {
-        const int id = s_out[i].id;
+        const int id = sm.kept_id[i];
         int rank = 0;
         for (int j = 0; j < kept; ++j) {
-            const int oj = s_out[j].id;
+            const int oj = sm.kept_id[j];
             rank += (oj < id || (oj == id && j < i)) ? 1 : 0;
         }
         sm.rank[i] = rank;
@@ -182,9 +182,9 @@ __device__ __forceinline__ void stage_finalize(const BatchDesc* __restrict__ b, 
         const int i = k / kWords, w = k - i * kWords;
         uint32_t v = 0;
         if (w < kDecodeWords) {
-            v = reinterpret_cast<const uint32_t*>(&s_out[i])[w];
+            v = reinterpret_cast<const uint32_t*>(&s_in[sm.kept_in[i]])[w];
         } else if (w > kDecodeWords) {
-            v = __float_as_uint(sm.h[sm.out_in[i]][w - kDecodeWords - 1]);
+            v = __float_as_uint(sm.h[sm.kept_in[i]][w - kDecodeWords - 1]);
         }
         words[sm.rank[i] * kWords + w] = v;
     }

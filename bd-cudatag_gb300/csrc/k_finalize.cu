@@ -18,10 +18,12 @@ std::atomic<int> g_fit_all_ctas_per_sm{1};
 
 int prepare_pipeline() {
     // Shared memory beyond 48 KB per block needs an opt-in, per device.
-    if (cudaFuncSetAttribute(k_binarize_runs, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(band_smem_bytes(kMaxBandCap, BD_MAX_WIDTH / 32))) !=
-        cudaSuccess) {
-        return -1;
+    for (int row_warps = 1; row_warps <= 2; ++row_warps) {
+        if (cudaFuncSetAttribute(binarize_kernel(row_warps), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(band_smem_bytes(kMaxBandCap, BD_MAX_WIDTH / 32))) !=
+            cudaSuccess) {
+            return -1;
+        }
     }
     if (cudaFuncSetAttribute(k_cand_count, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              static_cast<int>(cand_smem_bytes(kMaxBandsPerFrame))) != cudaSuccess) {
@@ -79,14 +81,27 @@ void enqueue_pipeline(const BatchDesc* dd, const BatchDesc& hd, const FrameIOArg
     mark(1);
     int words_max = 1;
     for (int f = 0; f < hd.frames; ++f) words_max = std::max(words_max, hd.f[f].words);
-    k_binarize_runs<<<bands, 256, band_smem_bytes(lc.band_cap, words_max), s>>>(dd, io, lc.band_cap,
-                                                                                 words_max);
+    // Threads per band.  Few bands (two per SM at most) leave the GPU's threads idle,
+    // and a band of a wide frame has several runs for each of 256: a 3840x2160 frame
+    // takes 62 us instead of 79 in k_binarize_runs with two warps per row (one lane per
+    // word is enough up to 1024 pixels: 640x480 loses 1), 44 instead of 61 in k_merge
+    // with 512 threads.  Many bands fill the GPU, and threads without a run then only hold
+    // others up: sixteen mixed frames take 65 us instead of 51 with two warps per row,
+    // 35 instead of 26 with 512 threads and 24 with 128; sixteen batches of four
+    // 1280x800 frames in flight gain 2% with 128.  Rows of more than 2048 pixels
+    // have runs for 256 (3840x2160: 111 us instead of 61 with 128).
+    const bool few_bands = bands <= 2 * sm_count;
+    const int row_warps = few_bands && words_max > 32 ? 2 : 1;
+    const int run_threads = few_bands ? 512 : (words_max > 64 ? 256 : 128);
+    const BinarizeKernel binarize = binarize_kernel(row_warps);
+    binarize<<<bands, 256 * row_warps, band_smem_bytes(lc.band_cap, words_max), s>>>(dd, io, lc.band_cap,
+                                                                                      words_max);
     mark(2);
     int row_cap_max = 1;
     for (int f = 0; f < hd.frames; ++f) row_cap_max = std::max(row_cap_max, hd.f[f].row_cap);
-    k_merge<<<bands, 256, 2 * row_cap_max * sizeof(uint32_t), s>>>(dd, io, row_cap_max);
+    k_merge<<<bands, run_threads, 2 * row_cap_max * sizeof(uint32_t), s>>>(dd, io, row_cap_max);
     mark(3);
-    k_region_stats<<<bands, 256, 0, s>>>(dd, io);
+    k_region_stats<<<bands, run_threads, 0, s>>>(dd, io);
     mark(4);
     const int split = lc.quad_split;
     int th_max = 1;

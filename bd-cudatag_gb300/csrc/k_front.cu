@@ -25,17 +25,21 @@ __global__ void __launch_bounds__(256) k_stats(const BatchDesc* __restrict__ b,
     stage_stats(b, frame, fi, blockIdx.x - b->stats_prefix[fi], sm);
 }
 
-__global__ void __launch_bounds__(256, 6) k_binarize_runs(const BatchDesc* __restrict__ b,
-                                                       const FrameIO* __restrict__ io, int cap,
-                                                       int bits_words) {
+// kRowWarps warps per row; the registers leave room for 48 warps per SM.
+template <int kRowWarps>
+__global__ void __launch_bounds__(256 * kRowWarps, 6 / kRowWarps)
+    k_binarize_runs(const BatchDesc* __restrict__ b, const FrameIO* __restrict__ io, int cap, int bits_words) {
     extern __shared__ __align__(16) uint32_t s_dyn[];
     __shared__ BinSmem sm;
     const int fi = frame_of_band(b, blockIdx.x);
     if (!io[fi].gray) return;
-    stage_binarize(b, io, fi, blockIdx.x - b->band_prefix[fi], cap, bits_words, sm, s_dyn);
+    stage_binarize<kRowWarps>(b, io, fi, blockIdx.x - b->band_prefix[fi], cap, bits_words, sm, s_dyn);
+}
+BinarizeKernel binarize_kernel(int row_warps) {
+    return row_warps == 2 ? k_binarize_runs<2> : k_binarize_runs<1>;
 }
 
-__global__ void __launch_bounds__(256, 2) k_merge(const BatchDesc* __restrict__ b,
+__global__ void __launch_bounds__(512, 2) k_merge(const BatchDesc* __restrict__ b,
                                                const FrameIO* __restrict__ io, int row_cap_max) {
     extern __shared__ __align__(16) uint32_t s_dyn[];
     const int fi = frame_of_band(b, blockIdx.x);
@@ -43,7 +47,7 @@ __global__ void __launch_bounds__(256, 2) k_merge(const BatchDesc* __restrict__ 
     stage_merge(b, fi, blockIdx.x - b->band_prefix[fi], row_cap_max, s_dyn);
 }
 
-__global__ void __launch_bounds__(256) k_region_stats(const BatchDesc* __restrict__ b,
+__global__ void __launch_bounds__(512) k_region_stats(const BatchDesc* __restrict__ b,
                                                       const FrameIO* __restrict__ io) {
     const int fi = frame_of_band(b, blockIdx.x);
     if (!io[fi].gray) return;

@@ -222,7 +222,7 @@ k_persistent(const BatchDesc* __restrict__ b, const FrameIO* __restrict__ io, Wo
                 break;
             }
             case kBin:
-                stage_binarize(b, io, fi, static_cast<int>(idx), band_cap, bits_words,
+                stage_binarize<1>(b, io, fi, static_cast<int>(idx), band_cap, bits_words,
                                *reinterpret_cast<BinSmem*>(dyn), reinterpret_cast<uint32_t*>(dyn + kBinDyn));
                 if (finish_unit(&st->done_bin, th, &ps.flag)) publish(b, q, kMerge, fi, th, false, &ps.base);
                 break;

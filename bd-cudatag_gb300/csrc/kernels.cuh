@@ -50,7 +50,8 @@ __host__ __device__ constexpr size_t cand_smem_bytes(int tile_h) {
 constexpr int kFinalThreads = 256;
 
 __global__ void k_stats(const BatchDesc* b, const __grid_constant__ FrameIOArgs io, FrameIO* io_out);
-__global__ void k_binarize_runs(const BatchDesc* b, const FrameIO* io, int cap, int bits_words);
+using BinarizeKernel = void (*)(const BatchDesc* b, const FrameIO* io, int cap, int bits_words);
+BinarizeKernel binarize_kernel(int row_warps);  // k_binarize_runs of 256 * row_warps threads: 1 or 2
 __global__ void k_merge(const BatchDesc* b, const FrameIO* io, int row_cap_max);
 __global__ void k_region_stats(const BatchDesc* b, const FrameIO* io);
 __global__ void k_cand_count(const BatchDesc* b, const FrameIO* io, int split_px);

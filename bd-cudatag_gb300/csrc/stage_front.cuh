@@ -3,8 +3,10 @@
 // band-local components, boundary unions, root aggregates, candidate
 // selection and ordering.  The per-stage kernels (k_front.cu) and the
 // persistent kernel (k_persistent.cu) both call them.  Every function
-// expects blockDim.x == 256 and takes its shared memory as a struct, so a
-// persistent kernel can overlay the stages' shared memory.  All FP32
+// takes its shared memory as a struct, so a persistent kernel can overlay the
+// stages' shared memory.  stage_stats and stage_cand expect blockDim.x == 256,
+// stage_binarize 256 * kRowWarps; stage_merge and stage_region take any whole
+// number of warps.  All FP32
 // arithmetic follows the reference expressions term by term and is compiled
 // with -fmad=false.
 #pragma once
@@ -31,6 +33,7 @@ struct BinSmem {
     uint8_t thresh[BD_MAX_WIDTH / kTile];
     uint8_t vmin[BD_MAX_WIDTH / kTile];
     uint8_t vmax[BD_MAX_WIDTH / kTile];
+    uint32_t warptot[32];      // fragments per warp, in pixel order
     uint32_t rowtot[kTile];
     uint32_t rowoff[kTile + 1];
     uint32_t nroots;
@@ -149,8 +152,8 @@ __device__ __forceinline__ void stage_stats(const BatchDesc* __restrict__ b, con
 
 // ===========================================================================
 // 2. Pooled threshold, binarization of the row band, run extraction and the
-//    band-local connected components, for one band of 8 rows; warp w owns
-//    row y0 + w.
+//    band-local connected components, for one band of 8 rows; kRowWarps
+//    warps per row (enqueue_pipeline says how many and why).
 //
 //    The runs of a band are labelled in shared memory (same-row fragments and
 //    8-connected runs of consecutive rows inside the band, by hooking and
@@ -168,6 +171,7 @@ __device__ __forceinline__ void stage_stats(const BatchDesc* __restrict__ b, con
 //    the band back to one root per run and full merging in k_merge.
 // ===========================================================================
 
+template <int kRowWarps>
 __device__ __forceinline__ void stage_binarize(const BatchDesc* __restrict__ b, const FrameIO* __restrict__ io, int fi,
                                int ty, int cap, int bits_words, BinSmem& sm, uint32_t* s_dyn) {
     uint32_t* sm_run = s_dyn;
@@ -258,21 +262,22 @@ __device__ __forceinline__ void stage_binarize(const BatchDesc* __restrict__ b, 
         if (mx - mn >= floor_contrast) thr = (mn + mx + 1) >> 1;
         s_thresh[t] = static_cast<uint8_t>(thr);
     }
-    if (tid < kTile) s_rowtot[tid] = 0;
     __syncthreads();
 
-    const int w = tid >> 5, lane = tid & 31;
+    const int warp = tid >> 5, lane = tid & 31;
+    const int w = warp / kRowWarps;                         // row
+    const int rl = (warp % kRowWarps) * 32 + lane;          // lane of the row's kRowWarps warps
     const uint8_t* gray = io[fi].gray;
     const int64_t stride = io[fi].stride;
     const bool vec = ((reinterpret_cast<uintptr_t>(gray) | static_cast<uintptr_t>(stride)) & 15u) == 0;
-    const int per = (words + 31) >> 5;
-    const int c0 = lane * per;
+    const int per = (words + 32 * kRowWarps - 1) / (32 * kRowWarps);
+    const int c0 = rl * per;
     const int c1 = min(c0 + per, words);
     uint32_t first_index = 0;  // exclusive prefix of this lane's fragments in its row
     if (w < rows) {
         const int y = y0 + w;
         const uint8_t* row = gray + static_cast<int64_t>(y) * stride;
-        for (int wx = lane; wx < words; wx += 32) {
+        for (int wx = rl; wx < words; wx += 32 * kRowWarps) {
             uint32_t m = 0xffffffffu;
             if (wx >= wx_lo && wx <= wx_hi) {
                 const int x = wx << 5;
@@ -298,8 +303,10 @@ __device__ __forceinline__ void stage_binarize(const BatchDesc* __restrict__ b, 
             d.bits[static_cast<int64_t>(y) * words + wx] = m;
             sm_bits[w * bits_words + wx] = m;
         }
-        __syncwarp();
-        // Fragments per lane, then the row's prefix (reference :448-470).
+    }
+    if (kRowWarps == 1) __syncwarp(); else __syncthreads();
+    if (w < rows) {
+        // Fragments per lane, then the warp's prefix (reference :448-470).
         uint32_t cnt = 0;
         for (int c = c0; c < c1; ++c) {
             const uint32_t m = sm_bits[w * bits_words + c];
@@ -311,29 +318,39 @@ __device__ __forceinline__ void stage_binarize(const BatchDesc* __restrict__ b, 
             if (lane >= off) incl += n;
         }
         first_index = incl - cnt;
-        const uint32_t total = __shfl_sync(kFull, incl, 31);
-        if (lane == 0) {
-            const uint32_t kept = min(total, row_cap);
-            d.row_count[y] = kept;
-            s_rowtot[w] = kept;
-        }
+        if (lane == 31) sm.warptot[warp] = incl;
+    } else if (lane == 31) {
+        sm.warptot[warp] = 0;
     }
     __syncthreads();
-    if (tid == 0) {
-        uint32_t off = 0;
-        for (int r = 0; r < kTile; ++r) {
-            s_rowoff[r] = off;
-            off += s_rowtot[r];
+    if (warp == 0) {
+        // Row totals and their prefix, by the lanes of one warp.
+        uint32_t kept = 0;
+        if (lane < kTile) {
+            for (int k = 0; k < kRowWarps; ++k) kept += sm.warptot[lane * kRowWarps + k];
+            kept = min(kept, row_cap);
+            s_rowtot[lane] = kept;
+            if (lane < rows) d.row_count[y0 + lane] = kept;
         }
-        s_rowoff[kTile] = off;
-        sm.nroots = 0;
-        atomicAdd(&st->counts[2], off);
+        uint32_t incl = kept;
+        for (int off = 1; off < kTile; off <<= 1) {
+            const uint32_t n = __shfl_up_sync(kFull, incl, off);
+            if (lane >= off) incl += n;
+        }
+        if (lane < kTile) s_rowoff[lane + 1] = incl;
+        if (lane == 0) s_rowoff[0] = 0;
+        if (lane == kTile - 1) atomicAdd(&st->counts[2], incl);
+        if (lane == 0) sm.nroots = 0;
+        __syncwarp();
+    }
+    if (tid == 0) {
         // Row segments that fit `cap` runs: a segment starts at row r > 0
         // (bit r) where adding row r would exceed the cap.  A row longer
         // than the cap by itself sends the band to the fallback.
         uint32_t mask = 0, cum = 0;
         bool fits = true;
-        for (int r = 0; r < kTile; ++r) {
+        const int cut_rows = s_rowoff[kTile] > static_cast<uint32_t>(cap) ? kTile : 0;
+        for (int r = 0; r < cut_rows; ++r) {
             const uint32_t n = s_rowtot[r];
             if (n > static_cast<uint32_t>(cap)) fits = false;
             if (cum > 0 && cum + n > static_cast<uint32_t>(cap)) {
@@ -355,6 +372,7 @@ __device__ __forceinline__ void stage_binarize(const BatchDesc* __restrict__ b, 
         const int y = y0 + w;
         const uint32_t slot_base = static_cast<uint32_t>(y) * row_cap;
         uint32_t index = first_index;
+        for (int k = w * kRowWarps; k < warp; ++k) index += sm.warptot[k];
         for (int c = c0; c < c1; ++c) {
             const uint32_t m = sm_bits[w * bits_words + c];
             d.word_first[static_cast<int64_t>(y) * words + c] = static_cast<uint16_t>(index);
@@ -427,7 +445,7 @@ __device__ __forceinline__ void stage_binarize(const BatchDesc* __restrict__ b, 
         // as long as the row, which every later find walks.  Row 0 of the
         // frame is never merged, not even its word-split fragments
         // (reference k_merge_runs :514 returns for y <= 0).
-        if (w >= r0 && w < r1 && w < rows && y0 + w > 0) {
+        if (rl < 32 && w >= r0 && w < r1 && w < rows && y0 + w > 0) {
             const uint32_t n = s_rowtot[w];
             const uint32_t base = s_rowoff[w] - seg_off;
             uint32_t carry = 0;  // group head of the previous chunk's last fragment
@@ -616,17 +634,19 @@ __device__ __forceinline__ void stage_merge(const BatchDesc* __restrict__ b, int
         }
         return;
     }
-    // Fallback band: every row, one warp per row.
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int y = ty * kTile + w;
-    if (y <= 0 || y >= d.height) return;
-    const int n = static_cast<int>(d.row_count[y]);
-    const int prev_n = static_cast<int>(d.row_count[y - 1]);
-    const uint32_t* cur = d.runs + static_cast<int64_t>(y) * row_cap;
-    const uint32_t* prev = d.runs + static_cast<int64_t>(y - 1) * row_cap;
-    for (int i = lane; i < n; i += 32) {
-        merge_run_with_row_above(parent, cur, prev, i, prev_n, static_cast<uint32_t>(y * row_cap),
-                                 static_cast<uint32_t>((y - 1) * row_cap), true);
+    // Fallback band: every row, a warp for each.
+    const int lane = threadIdx.x & 31;
+    for (int w = threadIdx.x >> 5; w < kTile; w += blockDim.x >> 5) {
+        const int y = ty * kTile + w;
+        if (y <= 0 || y >= d.height) continue;
+        const int n = static_cast<int>(d.row_count[y]);
+        const int prev_n = static_cast<int>(d.row_count[y - 1]);
+        const uint32_t* cur = d.runs + static_cast<int64_t>(y) * row_cap;
+        const uint32_t* prev = d.runs + static_cast<int64_t>(y - 1) * row_cap;
+        for (int i = lane; i < n; i += 32) {
+            merge_run_with_row_above(parent, cur, prev, i, prev_n, static_cast<uint32_t>(y * row_cap),
+                                     static_cast<uint32_t>((y - 1) * row_cap), true);
+        }
     }
 }
 

@@ -25,9 +25,10 @@ __global__ void __launch_bounds__(256) k_stats(const BatchDesc* __restrict__ b,
     stage_stats(b, frame, fi, blockIdx.x - b->stats_prefix[fi], sm);
 }
 
-// kRowWarps warps per row; the registers leave room for 48 warps per SM.
+// kRowWarps warps per row; the registers leave room for 48 warps per SM, or for
+// the two bands per SM that two warps per row are for.
 template <int kRowWarps>
-__global__ void __launch_bounds__(256 * kRowWarps, 6 / kRowWarps)
+__global__ void __launch_bounds__(256 * kRowWarps, kRowWarps == 1 ? 6 : 2)
     k_binarize_runs(const BatchDesc* __restrict__ b, const FrameIO* __restrict__ io, int cap, int bits_words) {
     extern __shared__ __align__(16) uint32_t s_dyn[];
     __shared__ BinSmem sm;

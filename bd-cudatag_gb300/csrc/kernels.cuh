@@ -34,11 +34,11 @@ namespace bdgb {
 
 constexpr int kMaxBandCap = 2048;
 // Dynamic shared memory of k_binarize_runs: six arrays of `cap` run
-// entries, the band's bit rows (kTile rows of `words` words), then the row
-// (byte) of each run entry.
+// entries, the band's bit rows (kTile rows of `words` words) and the runs
+// before each of their words (16 bits), then the row (byte) of each run entry.
 __host__ __device__ constexpr size_t band_smem_bytes(int cap, int words) {
-    return (6 * static_cast<size_t>(cap) + kTile * static_cast<size_t>(words)) * sizeof(uint32_t) +
-           static_cast<size_t>(cap);
+    return 6 * static_cast<size_t>(cap) * sizeof(uint32_t) +
+           kTile * static_cast<size_t>(words) * (sizeof(uint32_t) + sizeof(uint16_t)) + static_cast<size_t>(cap);
 }
 
 // Dynamic shared memory of k_cand_count: the candidates before each band (and

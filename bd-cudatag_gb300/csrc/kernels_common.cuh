@@ -46,6 +46,26 @@ __device__ __forceinline__ uint32_t white_bits4(uint32_t pixels, uint32_t t4) {
     return (((gt >> 7) & 0x01010101u) * 0x10204080u) >> 28;
 }
 
+// 4 * N bytes at p, of any alignment, from the aligned 32-bit words that hold them
+// (the last one only where a byte of it is asked for).
+template <int N>
+__device__ __forceinline__ void load_unaligned(const uint8_t* p, uint32_t (&v)[N]) {
+    const uint32_t off = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(p)) & 3u;
+    const uint32_t* q = reinterpret_cast<const uint32_t*>(p - off);
+    uint32_t w[N + 1];
+#pragma unroll
+    for (int k = 0; k < N; ++k) w[k] = __ldg(q + k);
+    w[N] = off ? __ldg(q + N) : 0u;
+#pragma unroll
+    for (int k = 0; k < N; ++k) v[k] = __funnelshift_r(w[k], w[k + 1], 8u * off);
+}
+
+// Whether load_unaligned of `bytes` bytes at pixel x of row y stays inside the
+// frame, from its first pixel to its last, gaps between rows included.
+__device__ __forceinline__ bool unaligned_inside(int x, int y, int bytes, int W, int H, int64_t stride) {
+    return (x > 0 || y > 0) && (x + bytes + 3 <= W || (y < H - 1 && x + bytes + 3 <= stride + W));
+}
+
 // ---------------------------------------------------------------------------
 // Tile statistics (reference k_tile_stats :104-135): min, max and rounded
 // mean of the 8x8 tiles of a frame.  One thread takes a pair of horizontally

@@ -181,7 +181,8 @@ __device__ __forceinline__ void stage_binarize(const BatchDesc* __restrict__ b, 
     uint32_t* sm_maxx = s_dyn + 4 * cap;
     uint32_t* sm_rows = s_dyn + 5 * cap;
     uint32_t* sm_bits = s_dyn + 6 * cap;  // kTile rows of bits_words words
-    uint8_t* sm_row = reinterpret_cast<uint8_t*>(sm_bits + kTile * bits_words);  // cap: row of each run
+    uint16_t* sm_first = reinterpret_cast<uint16_t*>(sm_bits + kTile * bits_words);  // runs before each word
+    uint8_t* sm_row = reinterpret_cast<uint8_t*>(sm_first + kTile * bits_words);     // cap: row of each run
     uint8_t* s_thresh = sm.thresh;
     uint8_t* s_vmin = sm.vmin;
     uint8_t* s_vmax = sm.vmax;
@@ -200,6 +201,29 @@ __device__ __forceinline__ void stage_binarize(const BatchDesc* __restrict__ b, 
     const int top = th - static_cast<int>(st->top_enc);
     const int bottom = static_cast<int>(st->bottom_enc) - 1;
     const bool on = bottom >= 0 && ty >= top - 1 && ty <= bottom + 1;
+    // The active columns and the column extremes of the three tile rows (all
+    // columns, to shared memory) are loaded ahead of the frame references, whose chain
+    // of reductions hides them.  (The first word of pixels as well: 53 us instead
+    // of 49 for sixteen mixed frames, its eight registers spill others.)
+    int lo = 0, hi = 0;
+    if (on) {
+        lo = d.row_lo[ty];
+        hi = d.row_hi[ty];
+        // The 3x3 window min/max, separably: columns over the three tile rows,
+        // then three columns.
+        for (int xx = tid; xx < tw; xx += blockDim.x) {
+            int mn = 255, mx = 0;
+#pragma unroll
+            for (int dy = -1; dy <= 1; ++dy) {
+                const int yy = ty + dy;
+                if (yy < 0 || yy >= th) continue;
+                mn = min(mn, static_cast<int>(d.tile_min[yy * tw + xx]));
+                mx = max(mx, static_cast<int>(d.tile_max[yy * tw + xx]));
+            }
+            s_vmin[xx] = static_cast<uint8_t>(mn);
+            s_vmax[xx] = static_cast<uint8_t>(mx);
+        }
+    }
     // Frame references from the complete histograms (reference
     // k_tile_reference :174-230): every band that thresholds computes them,
     // and band 0 also records them and the ROI row count (:2117).
@@ -225,7 +249,6 @@ __device__ __forceinline__ void stage_binarize(const BatchDesc* __restrict__ b, 
     }
 
     // Row band: contrasting tiles +- 4, or the whole row (reference :345-355).
-    const int lo = d.row_lo[ty], hi = d.row_hi[ty];
     const int start = lo < 0 ? 0 : max(0, lo - 4);
     const int end = lo < 0 ? tw - 1 : min(tw - 1, hi + 4);
     const int wx_lo = start >> 2;
@@ -235,21 +258,6 @@ __device__ __forceinline__ void stage_binarize(const BatchDesc* __restrict__ b, 
     const uint32_t ref0 = sm.refs[0], ref1 = sm.refs[1];
     const int floor_contrast = max(kMinTileContrast, static_cast<int>((ref0 * 3) / 2));
     const int t_end = min(4 * wx_hi + 3, tw - 1);
-    // The 3x3 window min/max, separably: columns over the three tile rows
-    // (coalesced loads into shared memory), then three columns.
-    const int c_lo = max(4 * wx_lo - 1, 0), c_hi = min(t_end + 1, tw - 1);
-    for (int xx = c_lo + tid; xx <= c_hi; xx += blockDim.x) {
-        int mn = 255, mx = 0;
-        for (int dy = -1; dy <= 1; ++dy) {
-            const int yy = ty + dy;
-            if (yy < 0 || yy >= th) continue;
-            mn = min(mn, static_cast<int>(d.tile_min[yy * tw + xx]));
-            mx = max(mx, static_cast<int>(d.tile_max[yy * tw + xx]));
-        }
-        s_vmin[xx] = static_cast<uint8_t>(mn);
-        s_vmax[xx] = static_cast<uint8_t>(mx);
-    }
-    __syncthreads();
     for (int t = 4 * wx_lo + tid; t <= t_end; t += blockDim.x) {
         int mn = 255, mx = 0;
         for (int dx = -1; dx <= 1; ++dx) {
@@ -280,17 +288,27 @@ __device__ __forceinline__ void stage_binarize(const BatchDesc* __restrict__ b, 
         for (int wx = rl; wx < words; wx += 32 * kRowWarps) {
             uint32_t m = 0xffffffffu;
             if (wx >= wx_lo && wx <= wx_hi) {
+                // A word is loaded whole in 16-byte-aligned rows, and in others from
+                // the aligned 32-bit words around it, wherever these lie inside the
+                // frame; byte by byte, a 1283x717 frame took 2 us more.
                 const int x = wx << 5;
-                if (vec && x + 32 <= W) {
-                    const uint4 a = *reinterpret_cast<const uint4*>(row + x);
-                    const uint4 c = *reinterpret_cast<const uint4*>(row + x + 16);
-                    const int t0 = x >> 3;
-                    const uint32_t q0 = s_thresh[t0] * 0x01010101u, q1 = s_thresh[t0 + 1] * 0x01010101u;
-                    const uint32_t q2 = s_thresh[t0 + 2] * 0x01010101u, q3 = s_thresh[t0 + 3] * 0x01010101u;
-                    m = white_bits4(a.x, q0) | (white_bits4(a.y, q0) << 4) |
-                        (white_bits4(a.z, q1) << 8) | (white_bits4(a.w, q1) << 12) |
-                        (white_bits4(c.x, q2) << 16) | (white_bits4(c.y, q2) << 20) |
-                        (white_bits4(c.z, q3) << 24) | (white_bits4(c.w, q3) << 28);
+                if (vec ? x + 32 <= W || (y < H - 1 && x + 32 <= stride + W)
+                        : unaligned_inside(x, y, 32, W, H, stride)) {
+                    m = 0u;
+#pragma unroll 1
+                    for (int half = 0; half < 32; half += 16) {
+                        __align__(16) uint32_t px[4];
+                        if (vec) {
+                            *reinterpret_cast<uint4*>(px) = *reinterpret_cast<const uint4*>(row + x + half);
+                        } else {
+                            load_unaligned(row + x + half, px);
+                        }
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            m |= white_bits4(px[k], s_thresh[((x + half) >> 3) + (k >> 1)] * 0x01010101u) << (4 * k + half);
+                        }
+                    }
+                    if (x + 32 > W) m |= ~((1u << (W - x)) - 1u);  // past the edge is white
                 } else {
                     m = 0u;
                     for (int k = 0; k < 32; ++k) {
@@ -376,6 +394,7 @@ __device__ __forceinline__ void stage_binarize(const BatchDesc* __restrict__ b, 
         for (int c = c0; c < c1; ++c) {
             const uint32_t m = sm_bits[w * bits_words + c];
             d.word_first[static_cast<int64_t>(y) * words + c] = static_cast<uint16_t>(index);
+            sm_first[w * bits_words + c] = static_cast<uint16_t>(index);
             uint32_t starts = ~m & ((m << 1) | 1u);
             const int last = min(31, W - 1 - (c << 5));
             while (starts) {
@@ -465,29 +484,23 @@ __device__ __forceinline__ void stage_binarize(const BatchDesc* __restrict__ b, 
         }
         // Then the rows meet: run i of row r > r0 overlaps (8-connected) the
         // runs [first, first + count) of row r - 1, kept in sm_area[i] until
-        // the roots pass needs it.
+        // the roots pass needs it.  The row's bits and the run counts before
+        // its words give both ends (runs do not cross words): two rounds of
+        // loads, where a search over the row's runs took seven.
         for (uint32_t i = tid; i < seg_n; i += blockDim.x) {
             const int row = sm_row[i];
             uint32_t list = 0;
             if (row > r0) {
                 const uint32_t run = sm_run[i];
-                const int x0 = static_cast<int>(run & 0xffffu);
-                const int x1 = static_cast<int>(run >> 16);
-                const uint32_t pbase = s_rowoff[row - 1] - seg_off;
-                const int prev_n = static_cast<int>(s_rowtot[row - 1]);
-                int lo2 = 0, hi2 = prev_n - 1, first = prev_n;
-                while (lo2 <= hi2) {
-                    const int mid = (lo2 + hi2) >> 1;
-                    if (static_cast<int>(sm_run[pbase + mid] >> 16) >= x0 - 1) {
-                        first = mid;
-                        hi2 = mid - 1;
-                    } else {
-                        lo2 = mid + 1;
-                    }
-                }
-                int k = first;
-                while (k < prev_n && static_cast<int>(sm_run[pbase + k] & 0xffffu) <= x1 + 1) ++k;
-                list = (pbase + static_cast<uint32_t>(first)) | (static_cast<uint32_t>(k - first) << 16);
+                const int xa = max(static_cast<int>(run & 0xffffu) - 1, 0);
+                const int xb = min(static_cast<int>(run >> 16) + 1, W - 1);
+                const int at_a = (row - 1) * bits_words + (xa >> 5), at_b = (row - 1) * bits_words + (xb >> 5);
+                const uint32_t ma = sm_bits[at_a], mb = sm_bits[at_b];
+                const uint32_t ends = ~ma & ((ma >> 1) | 0x80000000u);
+                const uint32_t starts = ~mb & ((mb << 1) | 1u);
+                const uint32_t first = sm_first[at_a] + __popc(ends & ((1u << (xa & 31)) - 1u));
+                const uint32_t past = sm_first[at_b] + __popc(starts & (kFull >> (31 - (xb & 31))));
+                list = (s_rowoff[row - 1] - seg_off + first) | ((past - first) << 16);
             }
             sm_area[i] = list;
         }

@@ -52,7 +52,8 @@ __global__ void __launch_bounds__(512) k_region_stats(const BatchDesc* __restric
                                                       const FrameIO* __restrict__ io) {
     const int fi = frame_of_band(b, blockIdx.x);
     if (!io[fi].gray) return;
-    stage_region(b, fi, blockIdx.x - b->band_prefix[fi]);
+    __shared__ RegionSmem sm;
+    stage_region(b, fi, blockIdx.x - b->band_prefix[fi], sm);
 }
 
 __global__ void __launch_bounds__(256) k_cand_count(const BatchDesc* __restrict__ b,

@@ -231,7 +231,7 @@ k_persistent(const BatchDesc* __restrict__ b, const FrameIO* __restrict__ io, Wo
                 if (finish_unit(&st->done_merge, th, &ps.flag)) publish(b, q, kRegion, fi, th, false, &ps.base);
                 break;
             case kRegion:
-                stage_region(b, fi, static_cast<int>(idx));
+                stage_region(b, fi, static_cast<int>(idx), *reinterpret_cast<RegionSmem*>(dyn));
                 if (finish_unit(&st->done_region, th, &ps.flag)) publish(b, q, kCand, fi, th, false, &ps.base);
                 break;
             case kCand: {
@@ -290,6 +290,7 @@ size_t persistent_smem_bytes(int band_cap, int bits_words, int row_cap_max, int 
     size_t bytes = sizeof(StatsSmem);
     bytes = std::max(bytes, kBinDyn + band_smem_bytes(band_cap, bits_words));
     bytes = std::max(bytes, 2 * static_cast<size_t>(row_cap_max) * sizeof(uint32_t));
+    bytes = std::max(bytes, sizeof(RegionSmem));
     bytes = std::max(bytes, kCandDyn + cand_smem_bytes(tile_h_max));
     bytes = std::max(bytes, kSmallPerUnit * sizeof(QuadSmem));
     bytes = std::max(bytes, sizeof(BigSmem));

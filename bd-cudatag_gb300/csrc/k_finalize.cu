@@ -81,18 +81,21 @@ void enqueue_pipeline(const BatchDesc* dd, const BatchDesc& hd, const FrameIOArg
     mark(1);
     int words_max = 1;
     for (int f = 0; f < hd.frames; ++f) words_max = std::max(words_max, hd.f[f].words);
-    // Threads per band.  Few bands (two per SM at most) leave the GPU's threads idle,
-    // and a band of a wide frame has several runs for each of 256: a 3840x2160 frame
-    // takes 62 us instead of 79 in k_binarize_runs with two warps per row (one lane per
-    // word is enough up to 1024 pixels: 640x480 loses 1), 44 instead of 61 in k_merge
-    // with 512 threads.  Many bands fill the GPU, and threads without a run then only hold
-    // others up: sixteen mixed frames take 65 us instead of 51 with two warps per row,
-    // 35 instead of 26 with 512 threads and 24 with 128; sixteen batches of four
-    // 1280x800 frames in flight gain 2% with 128.  Rows of more than 2048 pixels
-    // have runs for 256 (3840x2160: 111 us instead of 61 with 128).
+    // Threads per band.  A noisy band of a very wide frame has several runs for each
+    // of 256 threads, and a batch of few such bands (two per SM at most) leaves the GPU
+    // idle besides: a noisy 3840x2160 frame takes 62 us instead of 79 in
+    // k_binarize_runs with two warps per row, 44 instead of 61 in k_merge and 25
+    // instead of 31 in k_cand_count with 512 threads, and four such frames in flight lose 1%.
+    // Narrower ones gain 2 us at most alone and lose in flight (two 1600x1000
+    // frames 288 -> 303 us with two warps per row, 2560x1440 220 -> 229).
+    // Many bands of frames up to 2048 pixels wide leave most of 256 threads without a run
+    // in k_merge and k_region_stats: with 128, sixteen mixed frames take 24
+    // us instead of 26, and sixteen batches of four 1280x800 frames in flight gain 2%; few
+    // bands lose 2 us with 128, a noisy 3840x2160 frame 50.
     const bool few_bands = bands <= 2 * sm_count;
-    const int row_warps = few_bands && words_max > 32 ? 2 : 1;
-    const int run_threads = few_bands ? 512 : (words_max > 64 ? 256 : 128);
+    const bool more = few_bands && words_max > 96;  // wider than 3072 pixels
+    const int row_warps = more ? 2 : 1;
+    const int run_threads = more ? 512 : (!few_bands && words_max <= 64 ? 128 : 256);
     const BinarizeKernel binarize = binarize_kernel(row_warps);
     binarize<<<bands, 256 * row_warps, band_smem_bytes(lc.band_cap, words_max), s>>>(dd, io, lc.band_cap,
                                                                                       words_max);
@@ -106,7 +109,7 @@ void enqueue_pipeline(const BatchDesc* dd, const BatchDesc& hd, const FrameIOArg
     const int split = lc.quad_split;
     int th_max = 1;
     for (int f = 0; f < hd.frames; ++f) th_max = std::max(th_max, hd.f[f].tile_h);
-    k_cand_count<<<bands, 256, cand_smem_bytes(th_max), s>>>(dd, io, split);
+    k_cand_count<<<bands, more ? 512 : 256, cand_smem_bytes(th_max), s>>>(dd, io, split);
     mark(5);
     int cands = 0;
     for (int f = 0; f < hd.frames; ++f) cands += hd.f[f].max_candidates;

@@ -56,7 +56,7 @@ __global__ void __launch_bounds__(512) k_region_stats(const BatchDesc* __restric
     stage_region(b, fi, blockIdx.x - b->band_prefix[fi], sm);
 }
 
-__global__ void __launch_bounds__(256) k_cand_count(const BatchDesc* __restrict__ b,
+__global__ void __launch_bounds__(512) k_cand_count(const BatchDesc* __restrict__ b,
                                                     const FrameIO* __restrict__ io, int split_px) {
     extern __shared__ uint32_t s_dyn_cand[];  // cand_smem_bytes of the tallest frame
     __shared__ CandSmem sm;

@@ -4,9 +4,9 @@
 // selection and ordering.  The per-stage kernels (k_front.cu) and the
 // persistent kernel (k_persistent.cu) both call them.  Every function
 // takes its shared memory as a struct, so a persistent kernel can overlay the
-// stages' shared memory.  stage_stats and stage_cand expect blockDim.x == 256,
-// stage_binarize 256 * kRowWarps; stage_merge and stage_region take any whole
-// number of warps.  All FP32
+// stages' shared memory.  stage_stats expects blockDim.x == 256, stage_binarize
+// 256 * kRowWarps; stage_merge, stage_region and stage_cand take any whole number
+// of warps up to 16.  All FP32
 // arithmetic follows the reference expressions term by term and is compiled
 // with -fmad=false.
 #pragma once
@@ -49,7 +49,7 @@ struct CandSmem {
     uint32_t slot[kListCap];
     uint8_t bin[kListCap];
     uint32_t bins[kAreaBins];        // the band's candidates per bin; [0] all of them
-    uint32_t chunk[8][kAreaBins];
+    uint32_t chunk[16][kAreaBins];   // per warp
     uint32_t total[kAreaBins];
     uint32_t base[kAreaBins];
     uint32_t ncand, limit, nbig, nsmall;
@@ -914,8 +914,8 @@ __device__ __forceinline__ bool stage_cand(const BatchDesc* __restrict__ b, int 
     __threadfence();
 
     // Last band: the table into shared memory, eight loads in flight, then the
-    // exclusive prefix of every bin over the bands in place: warp q takes an eighth
-    // of the bands, lane = bin.  A prefix beyond 16 bits is cut to 65535:
+    // exclusive prefix of every bin over the bands in place: each warp takes a run
+    // of bands, lane = bin.  A prefix beyond 16 bits is cut to 65535:
     // such a candidate is past every cap either way.  Column 0 gives the candidates
     // before each band, in full.
     const int th = d.tile_h;
@@ -933,7 +933,8 @@ __device__ __forceinline__ bool stage_cand(const BatchDesc* __restrict__ b, int 
         }
     }
     __syncthreads();
-    const int per = (th + 7) >> 3;
+    const int warps = blockDim.x >> 5;
+    const int per = (th + warps - 1) / warps;
     const int b0 = min(th, w * per), b1 = min(th, b0 + per);
     uint32_t sum = 0;
 #pragma unroll 4
@@ -942,7 +943,7 @@ __device__ __forceinline__ bool stage_cand(const BatchDesc* __restrict__ b, int 
     __syncthreads();
     uint32_t carry = 0;
     for (int q = 0; q < w; ++q) carry += sm.chunk[q][lane];
-    if (w == 7) {
+    if (w == warps - 1) {
         sm.total[lane] = carry + sum;
         if (lane == 0) s_cprefix[th] = carry + sum;
     }

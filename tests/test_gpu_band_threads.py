@@ -21,6 +21,11 @@ def patterns(w, h):
     return out + [comb]
 
 
+@pytest.mark.parametrize("w,h,count", [(3072, 45, 3), (3073, 45, 3), (3840, 120, 3), (3105, 45, 64)])
+def test_wide_bands(w, h, count):
+    test_bands(w, h, count, 1024)
+
+
 @pytest.mark.parametrize("band_cap", [256, 2048])
 @pytest.mark.parametrize("w,h,count", [
     (1024, 45, 3), (1025, 45, 3), (1057, 45, 3), (2050, 45, 3),      # few bands

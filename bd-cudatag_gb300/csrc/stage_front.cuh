@@ -807,7 +807,7 @@ __device__ __forceinline__ uint32_t band_slot(const uint32_t* rowoff, int y0, ui
 // Bound: dependent L2 loads (two hops to the root, then area and box), then the
 // last CTA's chain.  Stage time (CUDA events, launch included): 18.4 -> 14.3 us
 // for four 1280x800 frames, 28.7 -> 20.5 for sixteen mixed ones, 51 -> 31 for
-// a noisy 3840x2160 frame (20 groups of runs a band).
+// a noisy 3840x2160 frame (20 groups of 256 runs a band), 25 with 512 threads.
 __device__ __forceinline__ bool stage_cand(const BatchDesc* __restrict__ b, int fi, int ty, int split_px, CandSmem& sm,
                            uint32_t* s_dyn) {
     uint32_t* s_rowoff = sm.rowoff;

@@ -193,7 +193,8 @@ BD_API int64_t bd_detector_debug_stage(bd_detector* detector, const char* name, 
  * bd_server_submit returns a ticket (>= 0), or BD_ERROR_OUT_OF_MEMORY when
  * the camera already has queue_depth frames waiting or running.  A frame in
  * page-locked host memory is read in place (keep it unchanged until its
- * ticket completes); other frames are copied at submit.  bd_server_wait /
+ * ticket completes); other frames are copied at submit, to device memory where
+ * the budget has room for it besides the plans.  bd_server_wait /
  * bd_server_poll return 1 with the results (out: 2 * max_detections records,
  * family-major; found[2], -1 for a family the camera does not decode;
  * latency_ms from submit to results), 0 from poll while pending, or a

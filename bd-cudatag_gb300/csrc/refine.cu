@@ -367,8 +367,10 @@ __global__ void __launch_bounds__(kGradWarps * 32, 2) k_refine_backward(bd_refin
 //
 // The photometric levels (mean intensity over the black and the white cells) are
 // not known before the samples are read.  The sums are taken against provisional levels (the last
-// iteration's; at first 0 and 255) and corrected by what the true ones differ from
-// them: one pass over the samples where there were two.
+// iteration's; at first those of a pass of their own) and corrected by what the true ones differ from
+// them: one pass over the samples where there were two.  The correction subtracts
+// FP32 sums, so it has to be small beside the residuals: where it is not, the
+// iteration's pass is taken again with the levels it found.
 //
 // Sample positions are relative to a whole pixel near the quad's centre: near
 // 1000 px they would carry 6e-5 px of rounding, and the parts of J^T J would
@@ -376,8 +378,9 @@ __global__ void __launch_bounds__(kGradWarps * 32, 2) k_refine_backward(bd_refin
 //
 // Bound: issue slots and L1 passes of the samples (some 100 instructions, 355
 // before), then the serial chain between two iterations (reduction, transform, FP64 solve: 40%).
-// 256 quads of 80 x 80 samples, 5 iterations: 792 us before, 120 us (170 us with 32
-// columns of one row to a warp).  Corners are five times nearer to 64-bit arithmetic.
+// 256 quads of 80 x 80 samples, 5 iterations: 792 us before, 131 us (50 us more with 32
+// columns of one row to a warp; 121 us from levels of 0 and 255 and without passes taken
+// again, but then the loss of the first pass is off by up to 2% at low contrast).
 // ---------------------------------------------------------------------------
 constexpr int kSums = 64;         // 61 used
 constexpr int kGnWarps = 10;      // 10 blocks of 8 columns: 10 cells of 8 samples (tag36h11)
@@ -417,6 +420,7 @@ struct GnSmem {
     float level[2];               // provisional: black, white
     int cx, cy;
     int ok;
+    int far;                      // the provisional levels were too far off
     GridSmem grid;
     float part[kGnWarps][kSums];
     float sum[kSums];
@@ -495,6 +499,96 @@ __device__ __forceinline__ bool solve8(double (&row)[8], double b, double lambda
     return true;
 }
 
+// A column of the sample grid, positions relative to a whole pixel near the centre.
+struct GnColumn {
+    float u, hx, hy, hd, h1, h4, h7;
+    uint32_t white_cells;
+};
+
+__device__ __forceinline__ GnColumn gn_column(const GnSmem& sm, const bd_refine_args& a, int col, int side) {
+    const int at = min(col, side - 1);
+    GnColumn c;
+    c.u = sm.grid.v[at];
+    c.white_cells = sm.grid.white[at / a.samples_per_cell];
+    c.hx = __fmaf_rn(sm.h[0], c.u, sm.h[2]);
+    c.hy = __fmaf_rn(sm.h[3], c.u, sm.h[5]);
+    c.hd = __fmaf_rn(sm.h[6], c.u, 1.0f);
+    c.h1 = sm.h[1];
+    c.h4 = sm.h[4];
+    c.h7 = sm.h[7];
+    return c;
+}
+
+// A sample of the column: its position, 1 / den, the 2 x 2 patch under it and the
+// value.  False outside the frame.
+struct GnSample {
+    float x, y, inv, fx, fy, dx_top, dx_bottom, top, bottom, value;
+};
+
+__device__ __forceinline__ bool gn_sample(const bd_refine_args& a, const uint8_t* __restrict__ image, int ox, int oy,
+                                          const GnColumn& c, float v, GnSample* s) {
+    const float den = __fmaf_rn(c.h7, v, c.hd);
+    s->inv = __frcp_rn(den);
+    s->x = __fmaf_rn(c.h1, v, c.hx) * s->inv;
+    s->y = __fmaf_rn(c.h4, v, c.hy) * s->inv;
+    const float fx0 = floorf(s->x), fy0 = floorf(s->y);
+    const int ix = static_cast<int>(fx0) + ox, iy = static_cast<int>(fy0) + oy;
+    if (!(den > 1e-6f) || static_cast<unsigned>(ix) >= static_cast<unsigned>(a.width - 1) ||
+        static_cast<unsigned>(iy) >= static_cast<unsigned>(a.height - 1)) {
+        return false;
+    }
+    s->fx = s->x - fx0;
+    s->fy = s->y - fy0;
+    const uint8_t* p = image + (static_cast<int64_t>(iy) * a.stride + ix);
+    const float pa = __ldg(p), pb = __ldg(p + 1);
+    const float pc = __ldg(p + a.stride), pd = __ldg(p + a.stride + 1);
+    s->dx_top = pb - pa;
+    s->dx_bottom = pd - pc;
+    s->top = __fmaf_rn(s->dx_top, s->fx, pa);
+    s->bottom = __fmaf_rn(s->dx_bottom, s->fx, pc);
+    s->value = __fmaf_rn(s->bottom - s->top, s->fy, s->top);
+    return true;
+}
+
+// Provisional levels of the first iteration: the mean value of each colour over a third of
+// the samples, which differs from the whole mean by less than the values do from
+// it (a colour without a sample keeps its level).  4 us of 131; all samples take 11.
+// Every thread; two barriers.
+__device__ __forceinline__ void gn_first_levels(GnSmem& sm, const bd_refine_args& a, const uint8_t* __restrict__ image,
+                                                int ox, int oy, const GridPlace& place, int side) {
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, warps = blockDim.x >> 5;
+    float total[4] = {};  // count and sum, black and white
+    for (int block = place.block0; block < place.blocks; block += warps) {
+        const int col = block * kTileCols + (lane & 7);
+        const GnColumn c = gn_column(sm, a, col, side);
+        for (int j = col < side ? place.row0 : side; j < side; j += 3 * place.row_step) {
+            GnSample s;
+            if (!gn_sample(a, image, ox, oy, c, sm.grid.v[j], &s)) continue;
+            const bool white = (c.white_cells & sm.grid.cell_bit[j]) != 0;
+            total[0] += white ? 0.0f : 1.0f;
+            total[1] += white ? 1.0f : 0.0f;
+            total[2] += white ? 0.0f : s.value;
+            total[3] += white ? s.value : 0.0f;
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) total[i] += __shfl_down_sync(0xffffffffu, total[i], off);
+        if (lane == 0) sm.part[warp][i] = total[i];
+    }
+    __syncthreads();
+    if (tid < 2) {
+        float count = 0.0f, sum = 0.0f;
+        for (int k = 0; k < warps; ++k) {
+            count += sm.part[k][tid];
+            sum += sm.part[k][tid + 2];
+        }
+        if (count > 0.0f) sm.level[tid] = sum / count;
+    }
+    __syncthreads();
+}
+
 __global__ void __launch_bounds__(kGnWarps * 32, 2) k_refine_gauss_newton(bd_refine_args a, float* corners,
                                                                      int iterations, float* loss) {
     __shared__ GnSmem sm;
@@ -514,7 +608,6 @@ __global__ void __launch_bounds__(kGnWarps * 32, 2) k_refine_gauss_newton(bd_ref
     load_grid(a, qi, sm.grid);
     const GridPlace place = grid_place(side);
     const int ox = sm.cx, oy = sm.cy;
-    const unsigned in_x = static_cast<unsigned>(a.width - 1), in_y = static_cast<unsigned>(a.height - 1);
 
     bool measured = false;  // the sums are those of a homography's samples
     for (int it = 0; it <= iterations; ++it) {
@@ -535,147 +628,150 @@ __global__ void __launch_bounds__(kGnWarps * 32, 2) k_refine_gauss_newton(bd_ref
         }
         __syncthreads();
         if (!sm.ok) break;
-        const float h1 = sm.h[1], h4 = sm.h[4], h7 = sm.h[7];
-        const float level_b = sm.level[0], level_w = sm.level[1];
-        for (int block = place.block0; block < place.blocks; block += warps) {
-            const int col = block * kTileCols + (lane & 7);
-            const float u = sm.grid.v[min(col, side - 1)];
-            const uint32_t white_cells = sm.grid.white[min(col, side - 1) / a.samples_per_cell];
-            const float hx = __fmaf_rn(sm.h[0], u, sm.h[2]);
-            const float hy = __fmaf_rn(sm.h[3], u, sm.h[5]);
-            const float hd = __fmaf_rn(sm.h[6], u, 1.0f);
-            float p0[6] = {}, p1[6] = {}, p2[6] = {};      // AA, BB, AB, AC, BC, CC by powers of v
-            float r0[3] = {}, r1[3] = {};                  // (A, B, C) r
-            float w0[3] = {}, w1[3] = {};                  // (A, B, C), white samples
-            float s0[3] = {}, s1[3] = {};                  // (A, B, C), all
-            float count[2] = {}, m1[2] = {}, m2[2] = {};
-            for (int j = col < side ? place.row0 : side; j < side; j += place.row_step) {
-                const float v = sm.grid.v[j];
-                const float den = __fmaf_rn(h7, v, hd);
-                const float inv = __frcp_rn(den);
-                const float x = __fmaf_rn(h1, v, hx) * inv;
-                const float y = __fmaf_rn(h4, v, hy) * inv;
-                const float fx0 = floorf(x), fy0 = floorf(y);
-                const int ix = static_cast<int>(fx0) + ox, iy = static_cast<int>(fy0) + oy;
-                if (!(den > 1e-6f) || static_cast<unsigned>(ix) >= in_x || static_cast<unsigned>(iy) >= in_y) continue;
-                const float fx = x - fx0, fy = y - fy0;
-                const uint8_t* p = image + (static_cast<int64_t>(iy) * a.stride + ix);
-                const float pa = __ldg(p), pb = __ldg(p + 1);
-                const float pc = __ldg(p + a.stride), pd = __ldg(p + a.stride + 1);
-                const float top = __fmaf_rn(pb - pa, fx, pa);
-                const float bottom = __fmaf_rn(pd - pc, fx, pc);
-                const float value = __fmaf_rn(bottom - top, fy, top);
-                const float A = __fmaf_rn((pd - pc) - (pb - pa), fy, pb - pa) * inv;
-                const float B = (bottom - top) * inv;
-                const float C = -__fmaf_rn(A, x, B * y);
-                const bool white = (white_cells & sm.grid.cell_bit[j]) != 0;
-                const float r = value - (white ? level_w : level_b);
-                const float vv = v * v;
-                const float pr[6] = {A * A, B * B, A * B, A * C, B * C, C * C};
+        if (it == 0 && !a.levels) gn_first_levels(sm, a, image, ox, oy, place, side);
+        for (bool first_pass = true;; first_pass = false) {
+            const float level_b = sm.level[0], level_w = sm.level[1];
+            for (int block = place.block0; block < place.blocks; block += warps) {
+                const int col = block * kTileCols + (lane & 7);
+                const GnColumn c = gn_column(sm, a, col, side);
+                const float u = c.u;
+                float p0[6] = {}, p1[6] = {}, p2[6] = {};      // AA, BB, AB, AC, BC, CC by powers of v
+                float r0[3] = {}, r1[3] = {};                  // (A, B, C) r
+                float w0[3] = {}, w1[3] = {};                  // (A, B, C), white samples
+                float s0[3] = {}, s1[3] = {};                  // (A, B, C), all
+                float count[2] = {}, m1[2] = {}, m2[2] = {};
+                for (int j = col < side ? place.row0 : side; j < side; j += place.row_step) {
+                    const float v = sm.grid.v[j];
+                    GnSample s;
+                    if (!gn_sample(a, image, ox, oy, c, v, &s)) continue;
+                    const float A = __fmaf_rn(s.dx_bottom - s.dx_top, s.fy, s.dx_top) * s.inv;
+                    const float B = (s.bottom - s.top) * s.inv;
+                    const float C = -__fmaf_rn(A, s.x, B * s.y);
+                    const bool white = (c.white_cells & sm.grid.cell_bit[j]) != 0;
+                    const float r = s.value - (white ? level_w : level_b);
+                    const float vv = v * v;
+                    const float pr[6] = {A * A, B * B, A * B, A * C, B * C, C * C};
 #pragma unroll
-                for (int i = 0; i < 6; ++i) {
-                    p0[i] += pr[i];
-                    p1[i] = __fmaf_rn(pr[i], v, p1[i]);
-                    p2[i] = __fmaf_rn(pr[i], vv, p2[i]);
+                    for (int i = 0; i < 6; ++i) {
+                        p0[i] += pr[i];
+                        p1[i] = __fmaf_rn(pr[i], v, p1[i]);
+                        p2[i] = __fmaf_rn(pr[i], vv, p2[i]);
+                    }
+                    const float abc[3] = {A, B, C};
+#pragma unroll
+                    for (int i = 0; i < 3; ++i) {
+                        const float ar = abc[i] * r;
+                        r0[i] += ar;
+                        r1[i] = __fmaf_rn(ar, v, r1[i]);
+                        s0[i] += abc[i];
+                        s1[i] = __fmaf_rn(abc[i], v, s1[i]);
+                        const float aw = white ? abc[i] : 0.0f;
+                        w0[i] += aw;
+                        w1[i] = __fmaf_rn(aw, v, w1[i]);
+                    }
+                    const float rw = white ? r : 0.0f, rb = white ? 0.0f : r;
+                    count[0] += white ? 0.0f : 1.0f;
+                    count[1] += white ? 1.0f : 0.0f;
+                    m1[0] += rb;
+                    m1[1] += rw;
+                    m2[0] = __fmaf_rn(rb, rb, m2[0]);
+                    m2[1] = __fmaf_rn(rw, rw, m2[1]);
                 }
-                const float abc[3] = {A, B, C};
+                // The column's u, then the sums over the CTA.
+                float sums[kSums] = {};
+                const float uu = u * u;
+                const int pair_at[3] = {kAA, kBB, kAB};
 #pragma unroll
                 for (int i = 0; i < 3; ++i) {
-                    const float ar = abc[i] * r;
-                    r0[i] += ar;
-                    r1[i] = __fmaf_rn(ar, v, r1[i]);
-                    s0[i] += abc[i];
-                    s1[i] = __fmaf_rn(abc[i], v, s1[i]);
-                    const float aw = white ? abc[i] : 0.0f;
-                    w0[i] += aw;
-                    w1[i] = __fmaf_rn(aw, v, w1[i]);
+                    sums[pair_at[i] + 0] = uu * p0[i];
+                    sums[pair_at[i] + 1] = u * p1[i];
+                    sums[pair_at[i] + 2] = u * p0[i];
+                    sums[pair_at[i] + 3] = p2[i];
+                    sums[pair_at[i] + 4] = p1[i];
+                    sums[pair_at[i] + 5] = p0[i];
                 }
-                const float rw = white ? r : 0.0f, rb = white ? 0.0f : r;
-                count[0] += white ? 0.0f : 1.0f;
-                count[1] += white ? 1.0f : 0.0f;
-                m1[0] += rb;
-                m1[1] += rw;
-                m2[0] = __fmaf_rn(rb, rb, m2[0]);
-                m2[1] = __fmaf_rn(rw, rw, m2[1]);
-            }
-            // The column's u, then the sums over the CTA.
-            float sums[kSums] = {};
-            const float uu = u * u;
-            const int pair_at[3] = {kAA, kBB, kAB};
 #pragma unroll
-            for (int i = 0; i < 3; ++i) {
-                sums[pair_at[i] + 0] = uu * p0[i];
-                sums[pair_at[i] + 1] = u * p1[i];
-                sums[pair_at[i] + 2] = u * p0[i];
-                sums[pair_at[i] + 3] = p2[i];
-                sums[pair_at[i] + 4] = p1[i];
-                sums[pair_at[i] + 5] = p0[i];
-            }
+                for (int i = 0; i < 2; ++i) {
+                    const int at = i == 0 ? kAC : kBC;
+                    sums[at + 0] = uu * p0[3 + i];
+                    sums[at + 1] = u * p1[3 + i];
+                    sums[at + 2] = u * p0[3 + i];
+                    sums[at + 3] = p2[3 + i];
+                    sums[at + 4] = p1[3 + i];
+                }
+                sums[kCC + 0] = uu * p0[5];
+                sums[kCC + 1] = u * p1[5];
+                sums[kCC + 2] = p2[5];
 #pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                const int at = i == 0 ? kAC : kBC;
-                sums[at + 0] = uu * p0[3 + i];
-                sums[at + 1] = u * p1[3 + i];
-                sums[at + 2] = u * p0[3 + i];
-                sums[at + 3] = p2[3 + i];
-                sums[at + 4] = p1[3 + i];
-            }
-            sums[kCC + 0] = uu * p0[5];
-            sums[kCC + 1] = u * p1[5];
-            sums[kCC + 2] = p2[5];
+                for (int i = 0; i < 3; ++i) {
+                    sums[kWR + 3 * i] = u * r0[i];
+                    sums[kWR + 3 * i + 1] = r1[i];
+                    sums[kWW + 3 * i] = u * w0[i];
+                    sums[kWW + 3 * i + 1] = w1[i];
+                    sums[kWAll + 3 * i] = u * s0[i];
+                    sums[kWAll + 3 * i + 1] = s1[i];
+                    if (i < 2) {
+                        sums[kWR + 3 * i + 2] = r0[i];
+                        sums[kWW + 3 * i + 2] = w0[i];
+                        sums[kWAll + 3 * i + 2] = s0[i];
+                    }
+                }
 #pragma unroll
-            for (int i = 0; i < 3; ++i) {
-                sums[kWR + 3 * i] = u * r0[i];
-                sums[kWR + 3 * i + 1] = r1[i];
-                sums[kWW + 3 * i] = u * w0[i];
-                sums[kWW + 3 * i + 1] = w1[i];
-                sums[kWAll + 3 * i] = u * s0[i];
-                sums[kWAll + 3 * i + 1] = s1[i];
-                if (i < 2) {
-                    sums[kWR + 3 * i + 2] = r0[i];
-                    sums[kWW + 3 * i + 2] = w0[i];
-                    sums[kWAll + 3 * i + 2] = s0[i];
+                for (int i = 0; i < 2; ++i) {
+                    sums[kCount + i] = count[i];
+                    sums[kMoment1 + i] = m1[i];
+                    sums[kMoment2 + i] = m2[i];
+                }
+                warp_sums(sums, lane);
+                const bool first = block == place.block0;
+                sm.part[warp][lane] = first ? sums[0] : sm.part[warp][lane] + sums[0];
+                sm.part[warp][lane + 32] = first ? sums[1] : sm.part[warp][lane + 32] + sums[1];
+            }
+            __syncthreads();
+            if (tid < kSums) {
+                float t = 0.0f;
+                for (int k = 0; k < warps; ++k) t += sm.part[k][tid];
+                sm.sum[tid] = t;
+            }
+            __syncthreads();
+            // T = W dH (entry (i, k) by thread 8 i + k); the true levels, as shifts
+            // of the provisional ones, by two threads of another warp.
+            if (tid < 64) {
+                const int i = tid >> 3, k = tid & 7;
+                float t = 0.0f;
+#pragma unroll
+                for (int m = 0; m < 8; ++m) t = __fmaf_rn(sm.sum[product_at(i, m)], sm.dh[m][k], t);
+                sm.t[i][k] = t;
+            } else if (tid < 66) {
+                const int i = tid - 64;
+                const bool own = !a.levels && sm.sum[kCount + i] > 0.0f;
+                sm.shift[i] = own ? sm.sum[kMoment1 + i] * reciprocal(sm.sum[kCount + i]) : 0.0;
+            }
+            if (warp == 2) {
+                __syncwarp();
+                if (lane < 8) {
+                    const double ww = sm.sum[kWW + lane];
+                    sm.wr[lane] = sm.sum[kWR + lane] - sm.shift[1] * ww - sm.shift[0] * (sm.sum[kWAll + lane] - ww);
+                } else if (lane == 8) {
+                    // A correction above the squared residuals would more than double the
+                    // rounding of their sum.  Below 2.5e-4 a level it is
+                    // lost in that of the values.  Some first steps exceed it: 6 us of 131.
+                    double moved = 0.0, left = 0.0;
+                    bool far = false;
+                    for (int i = 0; i < 2; ++i) {
+                        const double sh = sm.shift[i], n = sm.sum[kCount + i];
+                        moved += sh * sh * n;
+                        left += sm.sum[kMoment2 + i] - sh * (2.0 * sm.sum[kMoment1 + i] - sh * n);
+                        far = far || fabs(sh) > 2.5e-4;
+                    }
+                    sm.far = far && moved > left ? 1 : 0;
                 }
             }
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                sums[kCount + i] = count[i];
-                sums[kMoment1 + i] = m1[i];
-                sums[kMoment2 + i] = m2[i];
-            }
-            warp_sums(sums, lane);
-            const bool first = block == place.block0;
-            sm.part[warp][lane] = first ? sums[0] : sm.part[warp][lane] + sums[0];
-            sm.part[warp][lane + 32] = first ? sums[1] : sm.part[warp][lane + 32] + sums[1];
+            __syncthreads();
+            if (!first_pass || !sm.far) break;
+            if (tid < 2) sm.level[tid] = static_cast<float>(sm.level[tid] + sm.shift[tid]);
+            __syncthreads();
         }
-        __syncthreads();
-        if (tid < kSums) {
-            float t = 0.0f;
-            for (int k = 0; k < warps; ++k) t += sm.part[k][tid];
-            sm.sum[tid] = t;
-        }
-        __syncthreads();
-        // T = W dH (entry (i, k) by thread 8 i + k); the true levels, as shifts
-        // of the provisional ones, by two threads of another warp.
-        if (tid < 64) {
-            const int i = tid >> 3, k = tid & 7;
-            float t = 0.0f;
-#pragma unroll
-            for (int m = 0; m < 8; ++m) t = __fmaf_rn(sm.sum[product_at(i, m)], sm.dh[m][k], t);
-            sm.t[i][k] = t;
-        } else if (tid < 66) {
-            const int i = tid - 64;
-            const bool own = !a.levels && sm.sum[kCount + i] > 0.0f;
-            sm.shift[i] = own ? sm.sum[kMoment1 + i] * reciprocal(sm.sum[kCount + i]) : 0.0;
-        }
-        if (warp == 2) {
-            __syncwarp();
-            if (lane < 8) {
-                const double ww = sm.sum[kWW + lane];
-                sm.wr[lane] = sm.sum[kWR + lane] - sm.shift[1] * ww - sm.shift[0] * (sm.sum[kWAll + lane] - ww);
-            }
-        }
-        __syncthreads();
         if (warp == 0) {
             // Lane k (mod 8): row k of J^T J = dH^T T and of J^T r.
             if (it < iterations) {
@@ -713,7 +809,7 @@ __global__ void __launch_bounds__(kGnWarps * 32, 2) k_refine_gauss_newton(bd_ref
             const double sh = sm.shift[i];
             l += sm.sum[kMoment2 + i] - sh * (2.0 * sm.sum[kMoment1 + i] - sh * sm.sum[kCount + i]);
         }
-        loss[qi] = static_cast<float>(0.5 * l);
+        loss[qi] = static_cast<float>(l < 0.0 ? 0.0 : 0.5 * l);
     }
 }
 

@@ -348,7 +348,8 @@ __global__ void __launch_bounds__(kGradWarps * 32, 2) k_refine_backward(bd_refin
         for (int i = 0; i < 8; ++i) {
             float w = 0.0f;
             for (int k = 0; k < warps; ++k) w += s_part[k][i];
-            t = __fma_rn(static_cast<double>(w), static_cast<double>(s_dh[i][tid]), t);
+            // Without a sample in the frame the sums are 0 and dH may be anything.
+            if (w != 0.0f) t = __fma_rn(static_cast<double>(w), static_cast<double>(s_dh[i][tid]), t);
         }
         grad_corners[8 * qi + tid] = static_cast<float>(t);
     }

@@ -528,16 +528,17 @@ struct GnSample {
 
 __device__ __forceinline__ bool gn_sample(const bd_refine_args& a, const uint8_t* __restrict__ image, int ox, int oy,
                                           const GnColumn& c, float v, GnSample* s) {
+    // The frame's edges as seen from (ox, oy): whole numbers below 2^21, exact.
+    const float lo_x = static_cast<float>(-ox), hi_x = static_cast<float>(a.width - 1 - ox);
+    const float lo_y = static_cast<float>(-oy), hi_y = static_cast<float>(a.height - 1 - oy);
     const float den = __fmaf_rn(c.h7, v, c.hd);
     s->inv = __frcp_rn(den);
     s->x = __fmaf_rn(c.h1, v, c.hx) * s->inv;
     s->y = __fmaf_rn(c.h4, v, c.hy) * s->inv;
+    // In floats: a position that is no number or beyond an int's range is outside.
+    if (!(den > 1e-6f && s->x >= lo_x && s->x < hi_x && s->y >= lo_y && s->y < hi_y)) return false;
     const float fx0 = floorf(s->x), fy0 = floorf(s->y);
     const int ix = static_cast<int>(fx0) + ox, iy = static_cast<int>(fy0) + oy;
-    if (!(den > 1e-6f) || static_cast<unsigned>(ix) >= static_cast<unsigned>(a.width - 1) ||
-        static_cast<unsigned>(iy) >= static_cast<unsigned>(a.height - 1)) {
-        return false;
-    }
     s->fx = s->x - fx0;
     s->fy = s->y - fy0;
     const uint8_t* p = image + (static_cast<int64_t>(iy) * a.stride + ix);
@@ -600,8 +601,11 @@ __global__ void __launch_bounds__(kGnWarps * 32, 2) k_refine_gauss_newton(bd_ref
     const uint8_t* image = quad_image(a, qi);
     if (tid == 0) {
         const float* c = corners + 8 * qi;
-        sm.cx = static_cast<int>(floorf(0.25f * (c[0] + c[2] + c[4] + c[6])));
-        sm.cy = static_cast<int>(floorf(0.25f * (c[1] + c[3] + c[5] + c[7])));
+        // Kept below 2^20, far beyond any frame, so that the frame's edges stay exact
+        // (gn_sample); a NaN gives -2^20.
+        const float most = 1048576.0f;
+        sm.cx = static_cast<int>(fminf(fmaxf(floorf(0.25f * (c[0] + c[2] + c[4] + c[6])), -most), most));
+        sm.cy = static_cast<int>(fminf(fmaxf(floorf(0.25f * (c[1] + c[3] + c[5] + c[7])), -most), most));
         sm.level[0] = a.levels ? a.levels[2 * qi] : 0.0f;
         sm.level[1] = a.levels ? a.levels[2 * qi + 1] : 255.0f;
     }

@@ -1,6 +1,7 @@
 """Quads that are not there (gpu): corners that are not numbers, infinite or far outside
 beside one ordinary quad.  No sample of them lies in the frame: residuals, losses
-and gradients are 0, and the ordinary quad's results are those that it has alone.  All exact.
+and gradients are 0, Gauss-Newton leaves the corners as they are, and the
+ordinary quad's results are those that it has alone.  All exact.
 """
 import numpy as np
 import pytest
@@ -46,9 +47,26 @@ def gradients(corners):
     return [t.cpu().numpy() for t in (res, loss, gc)]
 
 
+def gauss_newton(corners):
+    image, co, templates = scene(corners)
+    loss = torch.full((len(corners),), -1.0, device="cuda")
+    args = bdcudatag.refine_args(image, co, templates, None, None, 8)
+    assert bdcudatag.lib().bd_refine_gauss_newton(args, co.data_ptr(), 3, loss.data_ptr(), None) == 0
+    torch.cuda.synchronize()
+    return co.cpu().numpy(), loss.cpu().numpy()
+
+
 @pytest.mark.parametrize("name", MISSING)
 def test_residuals_and_adjoint(name):
     both, alone = gradients([MISSING[name], QUAD]), gradients([QUAD])
     for got, want in zip(both, alone):
         assert np.all(got[0] == 0.0)
         assert np.array_equal(got[1], want[0])
+
+
+@pytest.mark.parametrize("name", MISSING)
+def test_gauss_newton(name):
+    (corners, loss), (want, want_loss) = gauss_newton([MISSING[name], QUAD]), gauss_newton([QUAD])
+    assert np.array_equal(corners[0], np.float32(MISSING[name]), equal_nan=True)
+    assert loss[0] == 0.0
+    assert np.array_equal(corners[1], want[0]) and loss[1] == want_loss[0]

@@ -26,6 +26,7 @@
 #include "bdcudatag/bdcudatag.h"
 #include "bdcudatag/bdcudatag_gb300.h"
 #include "families_data.inc"
+#include "reciprocal.h"
 
 namespace bdgb {
 void set_last_error(const char* message);  // capi.cpp
@@ -450,15 +451,6 @@ __device__ __forceinline__ int product_at(int i, int j) {
 
 __device__ __forceinline__ double shfl_double(double v, int lane) { return __shfl_sync(0xffffffffu, v, lane); }
 
-// 1 / d for d > 0 in float's range: Newton steps from the float reciprocal (24
-// good bits, then 48, then all).  FP64 is narrow on this GPU: a division is
-// twice as many of its instructions.
-__device__ __forceinline__ double reciprocal(double d) {
-    double r = static_cast<double>(__frcp_rn(static_cast<float>(d)));
-    r = __fma_rn(r, __fma_rn(-d, r, 1.0), r);
-    return __fma_rn(r, __fma_rn(-d, r, 1.0), r);
-}
-
 // One warp: (M + lambda diag(M)) x = -b by LDL^T in FP64, lane i = row i (lanes 8
 // and up repeat lanes 0-7).  False when a pivot is not positive.
 __device__ __forceinline__ bool solve8(double (&row)[8], double b, double lambda, int lane, double (*l_out)[8],
@@ -475,7 +467,7 @@ __device__ __forceinline__ bool solve8(double (&row)[8], double b, double lambda
     for (int j = 0; j < 8; ++j) {
         const double pivot = shfl_double(row[j], j);
         good = good && pivot > 1e-12;
-        const double inv = reciprocal(pivot);
+        const double inv = bdmath::reciprocal(pivot);
         if (i == j) inv_own = inv;
         const double l = row[j] * inv;
         const double yj = shfl_double(y, j);
@@ -750,7 +742,7 @@ __global__ void __launch_bounds__(kGnWarps * 32, 2) k_refine_gauss_newton(bd_ref
             } else if (tid < 66) {
                 const int i = tid - 64;
                 const bool own = !a.levels && sm.sum[kCount + i] > 0.0f;
-                sm.shift[i] = own ? sm.sum[kMoment1 + i] * reciprocal(sm.sum[kCount + i]) : 0.0;
+                sm.shift[i] = own ? sm.sum[kMoment1 + i] * bdmath::reciprocal(sm.sum[kCount + i]) : 0.0;
             }
             if (warp == 2) {
                 __syncwarp();

@@ -103,6 +103,24 @@ cudaError_t copy_pageable(uint8_t* dst, const uint8_t* src, int stride, int widt
     return queued != cudaSuccess ? queued : done;
 }
 
+// The plan's device made current while a call launches kernels or sets their
+// parameters: the caller's thread may have another one.
+class CurrentDevice {
+public:
+    explicit CurrentDevice(int device) {
+        int now = device;
+        if (cudaGetDevice(&now) == cudaSuccess && now != device && cudaSetDevice(device) == cudaSuccess) before_ = now;
+    }
+    ~CurrentDevice() {
+        if (before_ >= 0) cudaSetDevice(before_);
+    }
+    CurrentDevice(const CurrentDevice&) = delete;
+    CurrentDevice& operator=(const CurrentDevice&) = delete;
+
+private:
+    int before_ = -1;
+};
+
 struct Plan::Impl {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -514,6 +532,7 @@ uint8_t* Plan::host_frame(int i) { return impl_->frames_pinned + impl_->frame_of
 
 int Plan::submit_host(const uint8_t* const* frames, const int32_t* strides, std::string* error) {
     Impl& im = *impl_;
+    const CurrentDevice current(im.device);
     if (im.pending) {
         if (error) *error = "a batch is already in flight";
         return -1;
@@ -623,6 +642,7 @@ int Plan::submit_host(const uint8_t* const* frames, const int32_t* strides, std:
 
 int Plan::submit_device(const uint8_t* const* frames, const int32_t* strides, std::string* error) {
     Impl& im = *impl_;
+    const CurrentDevice current(im.device);
     if (im.pending) {
         if (error) *error = "a batch is already in flight";
         return -1;
@@ -650,6 +670,7 @@ int Plan::submit_device(const uint8_t* const* frames, const int32_t* strides, st
 
 int Plan::submit_slots(const uint8_t* const* frames, const int32_t* strides, std::string* error) {
     Impl& im = *impl_;
+    const CurrentDevice current(im.device);
     if (im.pending) {
         if (error) *error = "a batch is already in flight";
         return -1;

@@ -1,0 +1,70 @@
+"""Host paths that one GPU cannot show, against a stand-in for libcudart with two
+devices (cpp/fake_cudart.cpp; no GPU): the library in a process of its own, whose loader finds
+the stand-in first.
+"""
+import os
+import subprocess
+import sys
+import textwrap
+from pathlib import Path
+
+import pytest
+
+TESTS = Path(__file__).resolve().parent
+PKG = TESTS.parent / "bd-cudatag_gb300"
+CUDA = Path(os.environ.get("CUDA_HOME", "/usr/local/cuda"))
+
+PRELUDE = """
+import ctypes, sys, threading, time
+sys.path.insert(0, %r)
+import numpy as np
+import bdcudatag
+L = bdcudatag.lib()
+
+def device_frame(w, h):
+    p = ctypes.c_void_p()
+    assert L.cudaMalloc(ctypes.byref(p), ctypes.c_size_t(w * h)) == 0
+    return p.value
+
+def frame(w, h, first=0, pad=0):
+    f = np.zeros((h, w + pad), np.uint8)
+    f[0, 0] = first
+    return f
+""" % str(PKG)
+
+
+@pytest.fixture(scope="module")
+def stand_in(tmp_path_factory):
+    folder = tmp_path_factory.mktemp("cudart")
+    versions = folder / "versions"
+    versions.write_text("libcudart.so.13 { global: *; };\n")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-fPIC", "-shared", f"-I{CUDA / 'include'}",
+                    str(TESTS / "cpp" / "fake_cudart.cpp"), f"-Wl,--version-script={versions}",
+                    "-Wl,-soname,libcudart.so.13", "-o", str(folder / "libcudart.so.13"), "-lpthread"], check=True)
+    return folder
+
+
+def run(stand_in, script):
+    env = dict(os.environ, LD_LIBRARY_PATH=str(stand_in))
+    env.pop("LD_PRELOAD", None)
+    done = subprocess.run([sys.executable, "-c", PRELUDE + textwrap.dedent(script)], env=env, capture_output=True,
+                          text=True, timeout=120)
+    assert done.returncode == 0, done.stdout + done.stderr
+
+
+@pytest.mark.parametrize("graph", [0, 1])
+def test_other_current_device(stand_in, graph):
+    """A plan of device 0 called from a thread whose current device is 1: its graphs
+    run (no launches beside them), and the thread's device stays as it was."""
+    run(stand_in, f"""
+        batch = bdcudatag.Batch([(640, 480, 3), (320, 240, 1)], bdcudatag.default_config(use_cuda_graph={graph}))
+        server = bdcudatag.Server([(640, 480, 3)])
+        assert L.cudaSetDevice(1) == 0
+        for _ in range(3):
+            batch.detect([device_frame(640, 480), device_frame(320, 240)], [640, 320], device=True)
+            batch.detect([frame(640, 480), frame(320, 240)])
+            assert server.wait(server.submit(0, frame(640, 480)))[0] == 1
+        assert (L.fake_launches() == 0) == ({graph} == 1)
+        now = ctypes.c_int(-1)
+        assert L.cudaGetDevice(ctypes.byref(now)) == 0 and now.value == 1
+    """)

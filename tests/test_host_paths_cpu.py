@@ -68,3 +68,29 @@ def test_other_current_device(stand_in, graph):
         now = ctypes.c_int(-1)
         assert L.cudaGetDevice(ctypes.byref(now)) == 0 and now.value == 1
     """)
+
+
+def test_submits_do_not_wait_for_each_other(stand_in):
+    """While one thread's copy takes 400 ms, another camera's and another frame of the same
+    camera are submitted, and a copy that fails is reported by its own submit."""
+    run(stand_in, """
+        server = bdcudatag.Server([(1920, 1080, 1), (640, 480, 1)], queue_depth=4)
+        L.fake_slow(400)
+        slow, failing = frame(1920, 1080, first=200), frame(640, 480, first=100)
+        tickets = []
+        thread = threading.Thread(target=lambda: tickets.append(server.submit(0, slow)))
+        thread.start()
+        time.sleep(0.1)
+        for camera, f in ((1, frame(640, 480)), (0, frame(1920, 1080))):
+            before = time.perf_counter()
+            ticket = server.submit(camera, f)
+            assert time.perf_counter() - before < 0.2
+            assert ticket >= 0 and server.wait(ticket)[0] == 1
+        assert server.submit(1, failing) == bdcudatag.ERROR_CUDA
+        thread.join()
+        assert server.wait(tickets[0])[0] == 1
+        assert server.wait(server.submit(1, frame(640, 480)))[0] == 1
+        server.close()
+        assert L.fake_streams() == 0
+    """)
+

@@ -540,12 +540,9 @@ int Plan::submit_host(const uint8_t* const* frames, const int32_t* strides, std:
     const cudaStream_t s = im.active();
     // Frames in page-locked memory are copied by DMA straight from the caller,
     // and so are pageable ones where the GPU reads the host's page tables
-    // (figures at copy_pageable).  Rows with a gap are copied row by row, on which a small
-    // frame loses (300 KB: 28 us against 21 through staging memory; 1 MB: 47 to 72
-    // against 74; 8 MB: 134 against 644).  Others are compacted into the pinned
+    // (copies_direct, figures there and at copy_pageable).  Others are compacted into the pinned
     // staging buffer (the reference's detect_host path, gpu_detector.cu:2169-2176),
     // as is any pageable frame under a stream capture, whose replays read it there.
-    constexpr size_t kMinStridedCopy = 1 << 20;
     enum : uint8_t { kStaged, kPinned, kPageable };
     uint8_t source[kMaxFrames] = {};
     bool any_direct = false;
@@ -558,7 +555,6 @@ int Plan::submit_host(const uint8_t* const* frames, const int32_t* strides, std:
             return -1;
         }
         if (frames[i] == im.frames_pinned + im.frame_offset[i]) continue;  // already in the staging buffer
-        const size_t bytes = static_cast<size_t>(frames_[i].width) * frames_[i].height;
         cudaPointerAttributes attr;
         if (cudaPointerGetAttributes(&attr, frames[i]) != cudaSuccess) {
             cudaGetLastError();
@@ -567,7 +563,7 @@ int Plan::submit_host(const uint8_t* const* frames, const int32_t* strides, std:
         if (attr.type == cudaMemoryTypeHost) {
             source[i] = kPinned;
         } else if (attr.type == cudaMemoryTypeUnregistered && pageable &&
-                   (strides[i] == frames_[i].width || bytes >= kMinStridedCopy)) {
+                   copies_direct(strides[i], frames_[i].width, frames_[i].height)) {
             source[i] = kPageable;
         }
         any_direct = any_direct || source[i] != kStaged;

@@ -39,7 +39,7 @@ using Clock = std::chrono::steady_clock;
 
 // Takes the copy of a pageable frame: device memory where the GPU's copy engine reads
 // pageable frames and the budget holds the buffers besides the plans, page-locked
-// host memory otherwise.
+// host memory otherwise and for frames that do not go that way.
 struct RequestBuffer {
     uint8_t* device = nullptr;        // part of request_block, or null
     uint8_t* pinned = nullptr;
@@ -47,9 +47,13 @@ struct RequestBuffer {
 
 // Copies that go by the copy engine at once, each on a stream of its own: a submit
 // waits for its own copy and not for another thread's (a 640x480 camera beside three
-// threads with 3840x2160 frames: 100 us instead of 140 on one stream for all).  One
-// thread alone keeps to one stream: changing them costs 2 us a copy.
+// threads with 3840x2160 frames: 100 us instead of 140 on one stream for all, with gaps
+// between the rows 33 instead of 350).  One thread alone keeps to one stream: changing
+// them costs 2 us a copy.  Of rows with a gap the engine moves 92 GB/s in all and a
+// thread's memcpy 17, so from the fifth on a copy is sooner done by its own thread (eight
+// threads with 2560x1440 frames: 874 us a round with all of them on the engine, 735).
 constexpr size_t kDirectCopies = 8;
+constexpr int kStridedCopies = 4;
 
 struct Request {
     int camera = 0;
@@ -75,6 +79,7 @@ struct bd_server {
     std::vector<std::vector<RequestBuffer*>> free_buffers;
     uint8_t* request_block = nullptr;                // device memory of all buffers
     std::vector<cudaStream_t> free_streams;          // for copies to it; the last one is taken first
+    int strided_copies = 0;                          // in flight
     std::vector<int> outstanding;                    // per camera: requests not yet collected
     std::unordered_map<int64_t, Request> requests;
     int queue_depth = 0;
@@ -388,11 +393,15 @@ int64_t bd_server_submit(bd_server* s, int32_t camera, const uint8_t* gray, int3
         r.owned = s->free_buffers[camera].back();
         s->free_buffers[camera].pop_back();
         const RequestBuffer& b = *r.owned;
-        const bool direct = b.device && !s->free_streams.empty();
+        const bool strided = stride != cam.width;
+        const bool direct = b.device && !s->free_streams.empty() &&
+                            bdgb::copies_direct(stride, cam.width, cam.height) &&
+                            !(strided && s->strided_copies >= kStridedCopies);
         cudaStream_t stream = nullptr;
         if (direct) {
             stream = s->free_streams.back();
             s->free_streams.pop_back();
+            if (strided) ++s->strided_copies;
         }
         lock.unlock();
         cudaError_t copied = cudaSuccess;
@@ -407,6 +416,7 @@ int64_t bd_server_submit(bd_server* s, int32_t camera, const uint8_t* gray, int3
         lock.lock();
         if (direct) {
             s->free_streams.push_back(stream);
+            if (strided) --s->strided_copies;
         }
         if (copied != cudaSuccess) {
             s->free_buffers[camera].push_back(r.owned);

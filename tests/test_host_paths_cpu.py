@@ -94,3 +94,17 @@ def test_submits_do_not_wait_for_each_other(stand_in):
         assert L.fake_streams() == 0
     """)
 
+
+def test_strided_submits_to_a_server(stand_in):
+    """Rows with a gap: small frames through page-locked memory, as a batch takes them, large
+    ones by the copy engine."""
+    run(stand_in, """
+        server = bdcudatag.Server([(640, 480, 1), (1920, 1080, 1)])
+        L.fake_slow(300)
+        before = time.perf_counter()
+        assert server.wait(server.submit(0, frame(640, 480, first=200, pad=7), 647))[0] == 1
+        assert time.perf_counter() - before < 0.2  # the copy engine would have taken 300 ms
+        before = time.perf_counter()
+        assert server.wait(server.submit(1, frame(1920, 1080, first=200, pad=7), 1927))[0] == 1
+        assert time.perf_counter() - before >= 0.3
+    """)

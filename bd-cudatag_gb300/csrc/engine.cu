@@ -90,7 +90,7 @@ bool device_reads_pageable(int device) {
 }
 
 cudaError_t copy_pageable(uint8_t* dst, const uint8_t* src, int stride, int width, int height,
-                          cudaStream_t stream) {
+                          cudaStream_t stream, bool* refused) {
     // A capture that another thread has open in the global mode does not concern this stream.
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
     cudaThreadExchangeStreamCaptureMode(&mode);
@@ -98,9 +98,11 @@ cudaError_t copy_pageable(uint8_t* dst, const uint8_t* src, int stride, int widt
         stride == width
             ? cudaMemcpyAsync(dst, src, static_cast<size_t>(width) * height, cudaMemcpyDefault, stream)
             : cudaMemcpy2DAsync(dst, width, src, stride, width, height, cudaMemcpyDefault, stream);
-    const cudaError_t done = cudaStreamSynchronize(stream);
+    *refused = queued != cudaSuccess;
+    if (*refused) cudaGetLastError();
+    const cudaError_t done = *refused ? queued : cudaStreamSynchronize(stream);
     cudaThreadExchangeStreamCaptureMode(&mode);
-    return queued != cudaSuccess ? queued : done;
+    return done;
 }
 
 // The plan's device made current while a call launches kernels or sets their
@@ -570,13 +572,17 @@ int Plan::submit_host(const uint8_t* const* frames, const int32_t* strides, std:
     }
     cudaEventRecord(im.ev_start, s);
     // The pageable ones on the plan's own stream, which is idle here: the call
-    // waits for them, and not for what the caller's stream still has to do.
+    // waits for them, and not for what the caller's stream still has to do.  One that
+    // the runtime does not take goes through the staging buffer.
     if (any_direct) {
         for (int i = 0; i < this->frames(); ++i) {
             if (source[i] != kPageable) continue;
+            bool refused = false;
             const cudaError_t st = copy_pageable(im.frames_dev + im.frame_offset[i], frames[i], strides[i],
-                                                 frames_[i].width, frames_[i].height, im.stream);
-            if (st != cudaSuccess) {
+                                                 frames_[i].width, frames_[i].height, im.stream, &refused);
+            if (refused) {
+                source[i] = kStaged;
+            } else if (st != cudaSuccess) {
                 if (error) *error = cuda_error("cudaMemcpyAsync(frame)", st);
                 return -1;
             }

@@ -394,7 +394,7 @@ int64_t bd_server_submit(bd_server* s, int32_t camera, const uint8_t* gray, int3
         s->free_buffers[camera].pop_back();
         const RequestBuffer& b = *r.owned;
         const bool strided = stride != cam.width;
-        const bool direct = b.device && !s->free_streams.empty() &&
+        bool direct = b.device && !s->free_streams.empty() &&
                             bdgb::copies_direct(stride, cam.width, cam.height) &&
                             !(strided && s->strided_copies >= kStridedCopies);
         cudaStream_t stream = nullptr;
@@ -406,15 +406,21 @@ int64_t bd_server_submit(bd_server* s, int32_t camera, const uint8_t* gray, int3
         lock.unlock();
         cudaError_t copied = cudaSuccess;
         if (direct) {
-            copied = bdgb::copy_pageable(b.device, gray, stride, cam.width, cam.height, stream);
-        } else {
+            bool refused = false;
+            copied = bdgb::copy_pageable(b.device, gray, stride, cam.width, cam.height, stream, &refused);
+            if (refused) {
+                direct = false;
+                copied = cudaSuccess;
+            }
+        }
+        if (!direct) {
             for (int y = 0; y < cam.height; ++y) {
                 std::memcpy(b.pinned + static_cast<size_t>(y) * cam.width,
                             gray + static_cast<size_t>(y) * stride, cam.width);
             }
         }
         lock.lock();
-        if (direct) {
+        if (stream) {
             s->free_streams.push_back(stream);
             if (strided) --s->strided_copies;
         }

@@ -108,3 +108,22 @@ def test_strided_submits_to_a_server(stand_in):
         assert server.wait(server.submit(1, frame(1920, 1080, first=200, pad=7), 1927))[0] == 1
         assert time.perf_counter() - before >= 0.3
     """)
+
+
+def test_refused_copies_are_staged(stand_in):
+    """Pageable frames whose direct copy the runtime refuses go through page-locked memory, in
+    a batch beside a page-locked one and in a server; no error is left behind."""
+    run(stand_in, """
+        batch = bdcudatag.Batch([(640, 480, 3), (320, 240, 1), (640, 480, 1)])
+        server = bdcudatag.Server([(640, 480, 3)])
+        p = ctypes.c_void_p()
+        assert L.cudaHostAlloc(ctypes.byref(p), ctypes.c_size_t(640 * 480), 0) == 0
+        L.fake_refuse(1)
+        before = L.fake_copies_from_page_locked()
+        batch.detect([frame(640, 480), frame(320, 240), p.value], [640, 320, 640])
+        assert L.fake_copies_from_page_locked() == before + 3
+        for _ in range(20):  # streams are given back
+            assert server.wait(server.submit(0, frame(640, 480)))[0] == 1
+        assert L.fake_copies_from_page_locked() == before + 23
+        assert L.cudaGetLastError() == 0
+    """)

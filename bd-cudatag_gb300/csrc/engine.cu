@@ -570,6 +570,23 @@ int Plan::submit_host(const uint8_t* const* frames, const int32_t* strides, std:
         }
         any_direct = any_direct || source[i] != kStaged;
     }
+    auto stage = [&](int i) {
+        const int w = frames_[i].width, h = frames_[i].height;
+        uint8_t* dst = im.frames_pinned + im.frame_offset[i];
+        if (frames[i] == dst) return;
+        if (strides[i] == w) {
+            std::memcpy(dst, frames[i], static_cast<size_t>(w) * h);
+        } else {
+            for (int y = 0; y < h; ++y) {
+                std::memcpy(dst + static_cast<size_t>(y) * w,
+                            frames[i] + static_cast<size_t>(y) * strides[i], w);
+            }
+        }
+    };
+    for (int i = 0; i < this->frames(); ++i) {
+        if (source[i] == kStaged) stage(i);
+    }
+    // The batch's GPU time has the copies to the device in it, not the CPU's.
     cudaEventRecord(im.ev_start, s);
     // The pageable ones on the plan's own stream, which is idle here: the call
     // waits for them, and not for what the caller's stream still has to do.  One that
@@ -582,22 +599,10 @@ int Plan::submit_host(const uint8_t* const* frames, const int32_t* strides, std:
                                                  frames_[i].width, frames_[i].height, im.stream, &refused);
             if (refused) {
                 source[i] = kStaged;
+                stage(i);
             } else if (st != cudaSuccess) {
                 if (error) *error = cuda_error("cudaMemcpyAsync(frame)", st);
                 return -1;
-            }
-        }
-    }
-    for (int i = 0; i < this->frames(); ++i) {
-        const int w = frames_[i].width, h = frames_[i].height;
-        uint8_t* dst = im.frames_pinned + im.frame_offset[i];
-        if (source[i] != kStaged || frames[i] == dst) continue;
-        if (strides[i] == w) {
-            std::memcpy(dst, frames[i], static_cast<size_t>(w) * h);
-        } else {
-            for (int y = 0; y < h; ++y) {
-                std::memcpy(dst + static_cast<size_t>(y) * w,
-                            frames[i] + static_cast<size_t>(y) * strides[i], w);
             }
         }
     }

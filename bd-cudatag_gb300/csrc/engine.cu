@@ -558,15 +558,17 @@ int Plan::submit_host(const uint8_t* const* frames, const int32_t* strides, std:
         }
         if (frames[i] == im.frames_pinned + im.frame_offset[i]) continue;  // already in the staging buffer
         cudaPointerAttributes attr;
-        if (cudaPointerGetAttributes(&attr, frames[i]) != cudaSuccess) {
-            cudaGetLastError();
-            continue;
-        }
-        if (attr.type == cudaMemoryTypeHost) {
+        const bool known = cudaPointerGetAttributes(&attr, frames[i]) == cudaSuccess;
+        if (known && attr.type == cudaMemoryTypeHost) {
             source[i] = kPinned;
-        } else if (attr.type == cudaMemoryTypeUnregistered && pageable &&
-                   copies_direct(strides[i], frames_[i].width, frames_[i].height)) {
-            source[i] = kPageable;
+        } else {
+            // Also an error that an earlier call of this thread left behind: it is
+            // not this submit's.
+            cudaGetLastError();
+            if (known && attr.type == cudaMemoryTypeUnregistered && pageable &&
+                copies_direct(strides[i], frames_[i].width, frames_[i].height)) {
+                source[i] = kPageable;
+            }
         }
         any_direct = any_direct || source[i] != kStaged;
     }

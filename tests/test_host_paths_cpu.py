@@ -127,3 +127,14 @@ def test_refused_copies_are_staged(stand_in):
         assert L.fake_copies_from_page_locked() == before + 23
         assert L.cudaGetLastError() == 0
     """)
+
+
+def test_errors_of_earlier_calls(stand_in):
+    """An error that the caller's thread left behind does not fail a submit of pageable
+    frames."""
+    run(stand_in, """
+        batch = bdcudatag.Batch([(640, 480, 3), (320, 240, 1)])
+        for frames in ([frame(640, 480), frame(320, 240)], [frame(640, 480, pad=7), frame(320, 240, pad=7)]):
+            assert L.cudaSetDevice(99) != 0
+            batch.detect(frames)
+    """)

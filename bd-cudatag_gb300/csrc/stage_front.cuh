@@ -798,10 +798,52 @@ __device__ __forceinline__ uint32_t band_slot(const uint32_t* rowoff, int y0, ui
     return static_cast<uint32_t>(y0 + row) * row_cap + (i - rowoff[row]);
 }
 
+// Ranks of a band with more candidates than kListCap, and its list anew: the runs
+// once more in slot order, a thread each, the candidates before each by bin (column 0:
+// of any bin) counted per warp and carried on.  Comparing every pair took 133
+// us for 909 candidates of one band, this 31.  sm.total and sm.chunk are free here; every thread.
+__device__ __forceinline__ void rank_in_order(const FrameDesc& d, uint32_t* band_list, uint32_t* band_meta,
+                                              uint32_t total, int y0, int split_px, CandSmem& sm) {
+    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31, warps = blockDim.x >> 5;
+    if (tid < kAreaBins) sm.total[tid] = 0;
+    for (uint32_t base = 0; base < total; base += blockDim.x) {
+        const uint32_t i = base + tid;
+        uint32_t slot = 0;
+        int bin = -1;
+        bool big = false;
+        if (i < total) {
+            slot = band_slot(sm.rowoff, y0, static_cast<uint32_t>(d.row_cap), i);
+            if (__ldcg(d.parent + slot) == slot) bin = candidate_bin(d, slot, split_px, &big);
+        }
+        const uint32_t any = __ballot_sync(kFull, bin >= 0);
+        const uint32_t peers = __match_any_sync(kFull, bin) & any;
+        const uint32_t rank = __popc(peers & lanemask_lt());
+        sm.chunk[w][lane] = lane == 0 ? __popc(any) : 0u;
+        __syncwarp();
+        if (bin >= 0 && rank == 0) sm.chunk[w][bin - 32] = __popc(peers);
+        __syncthreads();
+        if (bin >= 0) {
+            uint32_t at = sm.total[0] + __popc(any & lanemask_lt());
+            uint32_t before = sm.total[bin - 32] + rank;
+            for (int q = 0; q < w; ++q) {
+                at += sm.chunk[q][0];
+                before += sm.chunk[q][bin - 32];
+            }
+            band_list[at] = slot;
+            band_meta[at] = (static_cast<uint32_t>(bin) << 24) | (big ? 1u << 23 : 0u) | before;
+        }
+        uint32_t add = 0;
+        for (int q = 0; tid < kAreaBins && q < warps; ++q) add += sm.chunk[q][lane];
+        __syncthreads();
+        if (tid < kAreaBins) sm.total[tid] += add;
+    }
+}
+
 // One CTA per band: root labels, the tag-like filter, and each candidate's
 // rank among the band's candidates of its area bin.  The candidates, a few of
 // thousands of runs, are listed as they come and ranked afterwards by
-// counting; ranking every 256 runs in order took four barriers a time.  The
+// counting; ranking every 256 runs in order took four barriers a time
+// (rank_in_order, for the bands with many).  The
 // frame's last CTA places the candidates.
 //
 // Bound: dependent L2 loads (two hops to the root, then area and box), then the
@@ -885,20 +927,15 @@ __device__ __forceinline__ bool stage_cand(const BatchDesc* __restrict__ b, int 
     __syncthreads();
     const uint32_t ncand = sm.ncand;
     const bool listed = ncand <= kListCap;
-    for (uint32_t c = tid; c < ncand; c += blockDim.x) {
-        const uint32_t slot = listed ? sm.slot[c] : __ldcg(band_list + c);
-        const uint32_t word = __ldcg(band_meta + c);
-        uint32_t rank = 0;
-        if (listed) {
-            const uint32_t bin = sm.bin[c];
+    if (listed) {
+        for (uint32_t c = tid; c < ncand; c += blockDim.x) {
+            const uint32_t slot = sm.slot[c], bin = sm.bin[c];
+            uint32_t rank = 0;
             for (uint32_t k = 0; k < ncand; ++k) rank += sm.bin[k] == bin && sm.slot[k] < slot ? 1u : 0u;
-        } else {
-            for (uint32_t k = 0; k < ncand; ++k) {
-                // Bin and slot only: other threads are adding the ranks.
-                rank += __ldcg(band_meta + k) >> 24 == word >> 24 && __ldcg(band_list + k) < slot ? 1u : 0u;
-            }
+            band_meta[c] = __ldcg(band_meta + c) | rank;
         }
-        band_meta[c] = word | rank;
+    } else {
+        rank_in_order(d, band_list, band_meta, total, y0, split_px, sm);
     }
     // The band's row of the candidate table: 16-bit counts per bin, [0] all.
     if (tid == 0) sm.bins[0] = ncand;  // bin 32 does not occur

@@ -26,7 +26,7 @@ int prepare_pipeline() {
         }
     }
     if (cudaFuncSetAttribute(k_cand_count, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(cand_smem_bytes(kMaxBandsPerFrame))) != cudaSuccess) {
+                             static_cast<int>(cand_smem_bytes(kMaxBandsPerFrame, kMaxBandsPerFrame))) != cudaSuccess) {
         return -1;
     }
     if (cudaFuncSetAttribute(k_fit_decode_all, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -107,9 +107,7 @@ void enqueue_pipeline(const BatchDesc* dd, const BatchDesc& hd, const FrameIOArg
     k_region_stats<<<bands, run_threads, 0, s>>>(dd, io);
     mark(4);
     const int split = lc.quad_split;
-    int th_max = 1;
-    for (int f = 0; f < hd.frames; ++f) th_max = std::max(th_max, hd.f[f].tile_h);
-    k_cand_count<<<bands, more ? 512 : 256, cand_smem_bytes(th_max), s>>>(dd, io, split);
+    k_cand_count<<<bands, more ? 512 : 256, cand_smem_bytes(hd), s>>>(dd, io, split);
     mark(5);
     int cands = 0;
     for (int f = 0; f < hd.frames; ++f) cands += hd.f[f].max_candidates;

@@ -284,14 +284,14 @@ k_persistent(const BatchDesc* __restrict__ b, const FrameIO* __restrict__ io, Wo
     }
 }
 
-size_t persistent_smem_bytes(int band_cap, int bits_words, int row_cap_max, int tile_h_max) {
+size_t persistent_smem_bytes(int band_cap, int bits_words, int row_cap_max, size_t cand_bytes) {
     constexpr size_t kBinDyn = (sizeof(BinSmem) + 15) / 16 * 16;
     constexpr size_t kCandDyn = (sizeof(CandSmem) + 15) / 16 * 16;
     size_t bytes = sizeof(StatsSmem);
     bytes = std::max(bytes, kBinDyn + band_smem_bytes(band_cap, bits_words));
     bytes = std::max(bytes, 2 * static_cast<size_t>(row_cap_max) * sizeof(uint32_t));
     bytes = std::max(bytes, sizeof(RegionSmem));
-    bytes = std::max(bytes, kCandDyn + cand_smem_bytes(tile_h_max));
+    bytes = std::max(bytes, kCandDyn + cand_bytes);
     bytes = std::max(bytes, kSmallPerUnit * sizeof(QuadSmem));
     bytes = std::max(bytes, sizeof(BigSmem));
     bytes = std::max(bytes, sizeof(FinalSmem));
@@ -303,7 +303,7 @@ size_t persistent_smem_bytes(int band_cap, int bits_words, int row_cap_max, int 
 int prepare_persistent() {
     // The largest overlay: band cap 2048 on the widest frame, tallest frame.
     const size_t most = persistent_smem_bytes(kMaxBandCap, BD_MAX_WIDTH / 32, BD_MAX_WIDTH / 2 + 2,
-                                              BD_MAX_HEIGHT / kTile);
+                                              cand_smem_bytes(kMaxBandsPerFrame, kMaxBandsPerFrame));
     return cudaFuncSetAttribute(k_persistent, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 static_cast<int>(most)) == cudaSuccess
                ? 0
@@ -313,13 +313,12 @@ int prepare_persistent() {
 void enqueue_persistent(const BatchDesc* dd, const BatchDesc& hd, const FrameIO* io, WorkQueue* queue,
                         void* stream_ptr, const LaunchConfig& lc, int sm_count, const PersistParams& pp) {
     cudaStream_t s = static_cast<cudaStream_t>(stream_ptr);
-    int words_max = 1, row_cap_max = 1, th_max = 1;
+    int words_max = 1, row_cap_max = 1;
     for (int f = 0; f < hd.frames; ++f) {
         words_max = std::max(words_max, hd.f[f].words);
         row_cap_max = std::max(row_cap_max, hd.f[f].row_cap);
-        th_max = std::max(th_max, hd.f[f].tile_h);
     }
-    const size_t smem = persistent_smem_bytes(lc.band_cap, words_max, row_cap_max, th_max);
+    const size_t smem = persistent_smem_bytes(lc.band_cap, words_max, row_cap_max, cand_smem_bytes(hd));
     int grid = lc.persist_ctas;
     if (grid <= 0) {
         int per_sm = 1;

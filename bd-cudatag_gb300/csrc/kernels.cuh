@@ -42,9 +42,26 @@ __host__ __device__ constexpr size_t band_smem_bytes(int cap, int words) {
 }
 
 // Dynamic shared memory of k_cand_count: the candidates before each band (and
-// in all), then the 32 16-bit counts of every band of the tallest frame.
-__host__ __device__ constexpr size_t cand_smem_bytes(int tile_h) {
-    return (static_cast<size_t>(tile_h) + 1) * sizeof(uint32_t) + static_cast<size_t>(tile_h) * 64;
+// in all) of the tallest frame, then the 32 16-bit counts of every band of the
+// tallest frame that has its table there: one of up to kTableBands.  The table costs every
+// CTA 64 bytes a band of residency (the persistent kernel's CTAs too), for the sake of
+// the frame's last one.  1280x8192: 41 us with it and 49 without.  Of 16384 rows, with it and
+// without: a frame of 1280 94 and 78, of noise 78 and 51, four of 1280 225 and 102, fifteen of
+// 640x480 and one of 64 88 and 51 (as persistent launch, the whole batch: 529 and 246).
+constexpr int kTableBands = 1024;
+__host__ __device__ constexpr size_t cand_smem_bytes(int tile_h, int table_h) {
+    return (static_cast<size_t>(tile_h) + 1) * sizeof(uint32_t) + static_cast<size_t>(table_h) * 64;
+}
+
+// The same for a batch.
+inline size_t cand_smem_bytes(const BatchDesc& hd) {
+    int tallest = 1, table = 0;
+    for (int f = 0; f < hd.frames; ++f) {
+        const int th = hd.f[f].tile_h;
+        if (th > tallest) tallest = th;
+        if (th <= kTableBands && th > table) table = th;
+    }
+    return cand_smem_bytes(tallest, table);
 }
 
 constexpr int kFinalThreads = 256;

@@ -839,6 +839,131 @@ __device__ __forceinline__ void rank_in_order(const FrameDesc& d, uint32_t* band
     }
 }
 
+// The frame's last CTA: prefixes of the candidate table (in shared memory, or where a
+// frame has more than kTableBands in place), then the candidates to their places.
+template <bool kShared>
+__device__ __forceinline__ void place_candidates(const FrameDesc& d, CandSmem& sm, uint32_t* s_dyn) {
+    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+    const uint32_t row_cap = static_cast<uint32_t>(d.row_cap);
+    FrameState* st = d.state;
+    // The table into shared memory, eight loads in flight, then the
+    // exclusive prefix of every bin over the bands in place: each warp takes a run
+    // of bands, lane = bin.  A prefix beyond 16 bits is cut to 65535:
+    // such a candidate is past every cap either way.  Column 0 gives the candidates
+    // before each band, in full.
+    const int th = d.tile_h;
+    uint32_t* s_cprefix = s_dyn;                                     // th + 1
+    uint32_t* s_words = s_dyn + th + 1;                              // th rows of 16 words
+    uint16_t* table = kShared ? reinterpret_cast<uint16_t*>(s_words) : reinterpret_cast<uint16_t*>(d.band_bins);
+    auto at_table = [&](int at) -> uint32_t { return kShared ? table[at] : __ldcg(table + at); };
+    const int words = kShared ? th * (kAreaBins / 2) : 0;
+    for (int i0 = tid; i0 < words; i0 += 8 * blockDim.x) {
+        uint32_t v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = i0 + k * blockDim.x < words ? __ldcg(&d.band_bins[i0 + k * blockDim.x]) : 0u;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            if (i0 + k * blockDim.x < words) s_words[i0 + k * blockDim.x] = v[k];
+        }
+    }
+    __syncthreads();
+    const int warps = blockDim.x >> 5;
+    const int per = (th + warps - 1) / warps;
+    const int b0 = min(th, w * per), b1 = min(th, b0 + per);
+    uint32_t sum = 0;
+#pragma unroll 4
+    for (int band = b0; band < b1; ++band) sum += at_table(band * kAreaBins + lane);
+    sm.chunk[w][lane] = sum;
+    __syncthreads();
+    uint32_t carry = 0;
+    for (int q = 0; q < w; ++q) carry += sm.chunk[q][lane];
+    if (w == warps - 1) {
+        sm.total[lane] = carry + sum;
+        if (lane == 0) s_cprefix[th] = carry + sum;
+    }
+    for (int band = b0; band < b1; band += 4) {
+        uint32_t n[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) n[k] = band + k < b1 ? at_table((band + k) * kAreaBins + lane) : 0u;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (band + k >= b1) break;
+            table[(band + k) * kAreaBins + lane] = static_cast<uint16_t>(min(carry, 0xffffu));
+            if (lane == 0) s_cprefix[band + k] = carry;
+            carry += n[k];
+        }
+    }
+    __syncthreads();
+    if (tid < 32) {
+        // Exclusive scan of the bin totals (column 0 is no bin).
+        const uint32_t t = lane == 0 ? 0u : sm.total[lane];
+        uint32_t incl = t;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const uint32_t n = __shfl_up_sync(kFull, incl, off);
+            if (lane >= off) incl += n;
+        }
+        sm.base[lane] = incl - t;
+        st->bin_base[lane] = 0;
+        st->bin_base[32 + lane] = incl - t;
+        if (lane == 31) {
+            st->counts[0] = incl;
+            sm.limit = min(incl, static_cast<uint32_t>(d.max_candidates));
+            st->n_candidates = sm.limit;
+            sm.nbig = 0;
+            sm.nsmall = 0;
+        }
+    }
+    __syncthreads();
+    // Placement (reference k_order_candidates :642-654): candidate j of the
+    // frame, flattened over the bands' lists, goes to bin base + earlier
+    // bands' count in its bin + its rank in the band.  Four candidates per thread and
+    // pass, their loads in flight together.
+    const uint32_t all = s_cprefix[th];
+    const uint32_t limit = sm.limit;
+    constexpr int kUnroll = 4;
+    for (uint32_t j0 = tid; j0 < all; j0 += kUnroll * blockDim.x) {
+        uint32_t slot[kUnroll], meta[kUnroll], prev[kUnroll];
+        int band[kUnroll];
+#pragma unroll
+        for (int u = 0; u < kUnroll; ++u) {
+            const uint32_t j = j0 + u * blockDim.x;
+            band[u] = -1;
+            if (j < all) {
+                int lo = 0, hi = th - 1;  // last band with s_cprefix[band] <= j
+                while (lo < hi) {
+                    const int mid = (lo + hi + 1) >> 1;
+                    if (s_cprefix[mid] <= j) lo = mid; else hi = mid - 1;
+                }
+                band[u] = lo;
+                const int64_t at = static_cast<int64_t>(lo) * kTile * row_cap + (j - s_cprefix[lo]);
+                slot[u] = __ldcg(&d.lroots[at]);
+                meta[u] = __ldcg(&d.cand_meta[at]);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kUnroll; ++u) {
+            prev[u] = band[u] < 0 ? 0u : at_table(band[u] * kAreaBins + static_cast<int>(meta[u] >> 24) - 32);
+        }
+#pragma unroll
+        for (int u = 0; u < kUnroll; ++u) {
+            if (band[u] < 0) continue;
+            const uint32_t pos = sm.base[(meta[u] >> 24) - 32u] + prev[u] + (meta[u] & 0x7fffffu);
+            if (pos < limit) {
+                d.candidates[pos] = slot[u];
+                // The fit/decode work lists, split by size once here: big
+                // candidates (a CTA each) from the front, the others (a warp
+                // per family) from the back.
+                if (meta[u] & (1u << 23)) {
+                    d.fit_list[atomicAdd(&sm.nbig, 1u)] = pos;
+                } else {
+                    d.fit_list[d.max_candidates - 1 - static_cast<int>(atomicAdd(&sm.nsmall, 1u))] = pos;
+                }
+            }
+        }
+    }
+}
+
 // One CTA per band: root labels, the tag-like filter, and each candidate's
 // rank among the band's candidates of its area bin.  The candidates, a few of
 // thousands of runs, are listed as they come and ranked afterwards by
@@ -950,112 +1075,10 @@ __device__ __forceinline__ bool stage_cand(const BatchDesc* __restrict__ b, int 
     if (!sm.last) return false;
     __threadfence();
 
-    // Last band: the table into shared memory, eight loads in flight, then the
-    // exclusive prefix of every bin over the bands in place: each warp takes a run
-    // of bands, lane = bin.  A prefix beyond 16 bits is cut to 65535:
-    // such a candidate is past every cap either way.  Column 0 gives the candidates
-    // before each band, in full.
-    const int th = d.tile_h;
-    uint32_t* s_cprefix = s_dyn;                                     // th + 1
-    uint32_t* s_words = s_dyn + th + 1;                              // th rows of 16 words
-    uint16_t* s_table = reinterpret_cast<uint16_t*>(s_words);
-    const int words = th * (kAreaBins / 2);
-    for (int i0 = tid; i0 < words; i0 += 8 * blockDim.x) {
-        uint32_t v[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) v[k] = i0 + k * blockDim.x < words ? __ldcg(&d.band_bins[i0 + k * blockDim.x]) : 0u;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            if (i0 + k * blockDim.x < words) s_words[i0 + k * blockDim.x] = v[k];
-        }
-    }
-    __syncthreads();
-    const int warps = blockDim.x >> 5;
-    const int per = (th + warps - 1) / warps;
-    const int b0 = min(th, w * per), b1 = min(th, b0 + per);
-    uint32_t sum = 0;
-#pragma unroll 4
-    for (int band = b0; band < b1; ++band) sum += s_table[band * kAreaBins + lane];
-    sm.chunk[w][lane] = sum;
-    __syncthreads();
-    uint32_t carry = 0;
-    for (int q = 0; q < w; ++q) carry += sm.chunk[q][lane];
-    if (w == warps - 1) {
-        sm.total[lane] = carry + sum;
-        if (lane == 0) s_cprefix[th] = carry + sum;
-    }
-#pragma unroll 4
-    for (int band = b0; band < b1; ++band) {
-        const uint32_t n = s_table[band * kAreaBins + lane];
-        s_table[band * kAreaBins + lane] = static_cast<uint16_t>(min(carry, 0xffffu));
-        if (lane == 0) s_cprefix[band] = carry;
-        carry += n;
-    }
-    __syncthreads();
-    if (tid < 32) {
-        // Exclusive scan of the bin totals (column 0 is no bin).
-        const uint32_t t = lane == 0 ? 0u : sm.total[lane];
-        uint32_t incl = t;
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const uint32_t n = __shfl_up_sync(kFull, incl, off);
-            if (lane >= off) incl += n;
-        }
-        sm.base[lane] = incl - t;
-        st->bin_base[lane] = 0;
-        st->bin_base[32 + lane] = incl - t;
-        if (lane == 31) {
-            st->counts[0] = incl;
-            sm.limit = min(incl, static_cast<uint32_t>(d.max_candidates));
-            st->n_candidates = sm.limit;
-            sm.nbig = 0;
-            sm.nsmall = 0;
-        }
-    }
-    __syncthreads();
-    // Placement (reference k_order_candidates :642-654): candidate j of the
-    // frame, flattened over the bands' lists, goes to bin base + earlier
-    // bands' count in its bin + its rank in the band.  Four candidates per thread and
-    // pass, their loads in flight together.
-    const uint32_t all = s_cprefix[th];
-    const uint32_t limit = sm.limit;
-    constexpr int kUnroll = 4;
-    for (uint32_t j0 = tid; j0 < all; j0 += kUnroll * blockDim.x) {
-        uint32_t slot[kUnroll], meta[kUnroll];
-        int band[kUnroll];
-#pragma unroll
-        for (int u = 0; u < kUnroll; ++u) {
-            const uint32_t j = j0 + u * blockDim.x;
-            band[u] = -1;
-            if (j < all) {
-                int lo = 0, hi = th - 1;  // last band with s_cprefix[band] <= j
-                while (lo < hi) {
-                    const int mid = (lo + hi + 1) >> 1;
-                    if (s_cprefix[mid] <= j) lo = mid; else hi = mid - 1;
-                }
-                band[u] = lo;
-                const int64_t at = static_cast<int64_t>(lo) * kTile * row_cap + (j - s_cprefix[lo]);
-                slot[u] = __ldcg(&d.lroots[at]);
-                meta[u] = __ldcg(&d.cand_meta[at]);
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < kUnroll; ++u) {
-            if (band[u] < 0) continue;
-            const uint32_t bin = (meta[u] >> 24) - 32u;
-            const uint32_t pos = sm.base[bin] + s_table[band[u] * kAreaBins + bin] + (meta[u] & 0x7fffffu);
-            if (pos < limit) {
-                d.candidates[pos] = slot[u];
-                // The fit/decode work lists, split by size once here: big
-                // candidates (a CTA each) from the front, the others (a warp
-                // per family) from the back.
-                if (meta[u] & (1u << 23)) {
-                    d.fit_list[atomicAdd(&sm.nbig, 1u)] = pos;
-                } else {
-                    d.fit_list[d.max_candidates - 1 - static_cast<int>(atomicAdd(&sm.nsmall, 1u))] = pos;
-                }
-            }
-        }
+    if (d.tile_h <= kTableBands) {
+        place_candidates<true>(d, sm, s_dyn);
+    } else {
+        place_candidates<false>(d, sm, s_dyn);
     }
     __syncthreads();
     if (tid == 0) {

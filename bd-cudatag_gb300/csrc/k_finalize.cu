@@ -84,25 +84,30 @@ void enqueue_pipeline(const BatchDesc* dd, const BatchDesc& hd, const FrameIOArg
     // Threads per band.  A noisy band of a very wide frame has several runs for each
     // of 256 threads, and a batch of few such bands (two per SM at most) leaves the GPU
     // idle besides: a noisy 3840x2160 frame takes 62 us instead of 79 in
-    // k_binarize_runs with two warps per row, 44 instead of 61 in k_merge and 25
-    // instead of 31 in k_cand_count with 512 threads, and four such frames in flight lose 1%.
-    // Narrower ones gain 2 us at most alone and lose in flight (two 1600x1000
+    // k_binarize_runs with two warps per row, and 25 instead of 31 in k_cand_count
+    // with 512 threads.  k_merge takes 512 only beyond 4096 pixels: in flight its larger
+    // CTAs cost more than they give alone (noise, alone and seven or so in flight: 3840x2160 126 and 455 us
+    // with 512 in k_merge, 132 and 386 with 256; 5120x2400 149 and 410, 159 and 369; 8192x2400
+    // 217 and 452, 277 and 480 with 256 in all).
+    // Narrower frames gain 2 us at most alone and lose in flight (two 1600x1000
     // frames 288 -> 303 us with two warps per row, 2560x1440 220 -> 229).
     // Many bands of frames up to 2048 pixels wide leave most of 256 threads without a run
     // in k_merge and k_region_stats: with 128, sixteen mixed frames take 24
-    // us instead of 26, and sixteen batches of four 1280x800 frames in flight gain 2%; few
+    // us instead of 26, and noisy batches in flight gain 5 to 15% (1280x800x4 436 -> 415,
+    // 1920x1080x5 412 -> 360; alone they lose up to 6%); few
     // bands lose 2 us with 128, a noisy 3840x2160 frame 50.
     const bool few_bands = bands <= 2 * sm_count;
     const bool more = few_bands && words_max > 96;  // wider than 3072 pixels
     const int row_warps = more ? 2 : 1;
     const int run_threads = more ? 512 : (!few_bands && words_max <= 64 ? 128 : 256);
+    const int merge_threads = more && words_max <= 128 ? 256 : run_threads;
     const BinarizeKernel binarize = binarize_kernel(row_warps);
     binarize<<<bands, 256 * row_warps, band_smem_bytes(lc.band_cap, words_max), s>>>(dd, io, lc.band_cap,
                                                                                       words_max);
     mark(2);
     int row_cap_max = 1;
     for (int f = 0; f < hd.frames; ++f) row_cap_max = std::max(row_cap_max, hd.f[f].row_cap);
-    k_merge<<<bands, run_threads, 2 * row_cap_max * sizeof(uint32_t), s>>>(dd, io, row_cap_max);
+    k_merge<<<bands, merge_threads, 2 * row_cap_max * sizeof(uint32_t), s>>>(dd, io, row_cap_max);
     mark(3);
     k_region_stats<<<bands, run_threads, 0, s>>>(dd, io);
     mark(4);
@@ -115,7 +120,10 @@ void enqueue_pipeline(const BatchDesc* dd, const BatchDesc& hd, const FrameIOArg
     // pixels, up to the three that fit.  With one, sixteen mixed frames (22 Mi, some 350
     // of them) took 76 us instead of 49 and a 3840x2160 frame 47 instead of 35; with
     // three for any batch, four 1280x800 frames with many batches in flight
-    // lost 1% to CTAs without work.
+    // lost 1% to CTAs without work.  The step itself is flat: up to 4.9 Mi (1280x800 to
+    // 1920x1080, two to five frames) one, two or three differ by 2% alone and in flight, and from
+    // 5.9 Mi on one loses alone (six 1280x800 135 instead of 120, four 1600x1200 140 instead of 121)
+    // and nothing in flight.
     int64_t pixels = 0;
     for (int f = 0; f < hd.frames; ++f) pixels += static_cast<int64_t>(hd.f[f].width) * hd.f[f].height;
     const int per_sm = static_cast<int>(std::min<int64_t>(3, (pixels + (4 << 20) - 1) / (4 << 20)));

@@ -544,7 +544,8 @@ int Plan::submit_host(const uint8_t* const* frames, const int32_t* strides, std:
     // and so are pageable ones where the GPU reads the host's page tables
     // (copies_direct, figures there and at copy_pageable).  Others are compacted into the pinned
     // staging buffer (the reference's detect_host path, gpu_detector.cu:2169-2176),
-    // as is any pageable frame under a stream capture, whose replays read it there.
+    // as is any pageable frame under a stream capture, whose replays read it there (a
+    // plan without graphs; one with graphs refuses to be captured).
     enum : uint8_t { kStaged, kPinned, kPageable };
     uint8_t source[kMaxFrames] = {};
     bool any_direct = false;

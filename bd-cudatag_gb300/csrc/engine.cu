@@ -150,8 +150,8 @@ struct Plan::Impl {
     uint8_t* results_pinned = nullptr;  // written by the GPU
     size_t results_bytes = 0;
     size_t result_stride = 0;
-    cudaGraphExec_t graph_host = nullptr;    // H2D of the staging buffer + pipeline + D2H
-    cudaGraphExec_t graph_fixed = nullptr;   // pipeline + D2H on the plan's device frames
+    cudaGraphExec_t graph_host = nullptr;    // H2D of the staging buffer + pipeline
+    cudaGraphExec_t graph_fixed = nullptr;   // pipeline on the plan's device frames
     cudaGraphExec_t graph_device = nullptr;  // caller device frames (first kernel's argument)
     cudaGraph_t graph_device_src = nullptr;  // holds stats_node
     cudaGraphNode_t stats_node = nullptr;

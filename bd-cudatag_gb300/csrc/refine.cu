@@ -20,7 +20,6 @@
 
 #include <cuda_runtime.h>
 
-#include <algorithm>
 #include <cstdint>
 
 #include "bdcudatag/bdcudatag.h"
@@ -398,7 +397,7 @@ enum SumAt {
     kCount = 55, kMoment1 = 57, kMoment2 = 59
 };
 
-// Sum over the lanes of a warp of each of 64 values: 63 shuffles (value pairs are
+// Sum over the lanes of a warp of each of 64 values: 62 shuffles (value pairs are
 // split between the halves of the warp, then the quarters ...) where a
 // tree per value takes 320.  Lane l is left with the sums of values l and l + 32 in
 // v[0] and v[1].
@@ -895,8 +894,8 @@ int32_t bd_refine_gauss_newton(const bd_refine_args* args, float* corners_inout,
         return BD_ERROR_INVALID_ARGUMENT;
     }
     if (args->count == 0) return BD_OK;
-    // At least the three warps that the steps between the samples use.
-    const int warps = std::max(3, grid_warps(args->cells * args->samples_per_cell, kGnWarps));
+    // 6 to 10 warps (3 to 256 samples a side); the steps between the samples use three.
+    const int warps = grid_warps(args->cells * args->samples_per_cell, kGnWarps);
     k_refine_gauss_newton<<<args->count, warps * 32, 0, static_cast<cudaStream_t>(cuda_stream)>>>(
         *args, corners_inout, iterations, loss);
     return launched();

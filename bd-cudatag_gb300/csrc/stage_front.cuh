@@ -1005,7 +1005,7 @@ __device__ __forceinline__ bool stage_cand(const BatchDesc* __restrict__ b, int 
     // cand_meta, for the frame's last CTA to place.
     uint32_t* band_list = d.lroots + static_cast<int64_t>(ty) * kTile * row_cap;
     uint32_t* band_meta = d.cand_meta + static_cast<int64_t>(ty) * kTile * row_cap;
-    // Up to four groups of 256 runs at a time, their label and root loads
+    // Up to four groups of a run per thread at a time, their label and root loads
     // issued together.
     constexpr int kChunks = 4;
     for (uint32_t gbase = 0; gbase < total; gbase += kChunks * blockDim.x) {

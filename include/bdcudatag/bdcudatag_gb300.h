@@ -61,7 +61,8 @@ BD_API int32_t bd_batch_detect_device(bd_batch* batch, const uint8_t* const* fra
                                       const int32_t* strides, bd_detection* out, int32_t* found);
 
 /* Split form of the calls above: submit enqueues the batch and returns at
- * once; wait blocks until it finishes and writes out / found.  One batch may
+ * once (frames in pageable host memory: when they have been copied, behind copies
+ * that are queued already); wait blocks until it finishes and writes out / found.  One batch may
  * be in flight per bd_batch; use several batches to overlap. */
 BD_API int32_t bd_batch_submit_host(bd_batch* batch, const uint8_t* const* frames,
                                     const int32_t* strides);

@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(kGradWarps * 32, 2) k_refine_backward(bd_refin
 //
 // The photometric levels (mean intensity over the black and the white cells) are
 // not known before the samples are read.  The sums are taken against provisional levels (the last
-// iteration's; at first those of a pass of their own) and corrected by what the true ones differ from
+// iteration's; at first those of a few samples) and corrected by what the true ones differ from
 // them: one pass over the samples where there were two.  The correction subtracts
 // FP32 sums, so it has to be small beside the residuals: where it is not, the
 // iteration's pass is taken again with the levels it found.
@@ -379,7 +379,7 @@ __global__ void __launch_bounds__(kGradWarps * 32, 2) k_refine_backward(bd_refin
 //
 // Bound: issue slots and L1 passes of the samples (some 100 instructions, 355
 // before), then the serial chain between two iterations (reduction, transform, FP64 solve: 40%).
-// 256 quads of 80 x 80 samples, 5 iterations: 792 us before, 131 us (50 us more with 32
+// 256 quads of 80 x 80 samples, 5 iterations: 792 us before, 124 us (50 us more with 32
 // columns of one row to a warp; 121 us from levels of 0 and 255 and without passes taken
 // again, but then the loss of the first pass is off by up to 2% at low contrast).  Error
 // against 64-bit arithmetic, twelve sets of such quads: 8.3e-7 before and 4.2e-7 in the corners, 4.1e-6
@@ -545,9 +545,9 @@ __device__ __forceinline__ bool gn_sample(const bd_refine_args& a, const uint8_t
     return true;
 }
 
-// Provisional levels of the first iteration: the mean value of each colour over a third of
+// Provisional levels of the first iteration: the mean value of each colour over a fifth of
 // the samples, which differs from the whole mean by less than the values do from
-// it (a colour without a sample keeps its level).  4 us of 131; all samples take 11.
+// it (a colour without a sample keeps its level).  2 us of 124; a third of them takes 4, all take 11.
 // Every thread; two barriers.
 __device__ __forceinline__ void gn_first_levels(GnSmem& sm, const bd_refine_args& a, const uint8_t* __restrict__ image,
                                                 int ox, int oy, const GridPlace& place, int side) {
@@ -556,7 +556,7 @@ __device__ __forceinline__ void gn_first_levels(GnSmem& sm, const bd_refine_args
     for (int block = place.block0; block < place.blocks; block += warps) {
         const int col = block * kTileCols + (lane & 7);
         const GnColumn c = gn_column(sm, a, col, side);
-        for (int j = col < side ? place.row0 : side; j < side; j += 3 * place.row_step) {
+        for (int j = col < side ? place.row0 : side; j < side; j += 5 * place.row_step) {
             GnSample s;
             if (!gn_sample(a, image, ox, oy, c, sm.grid.v[j], &s)) continue;
             const bool white = (c.white_cells & sm.grid.cell_bit[j]) != 0;
@@ -601,6 +601,7 @@ __global__ void __launch_bounds__(kGnWarps * 32, 2) k_refine_gauss_newton(bd_ref
         sm.cy = static_cast<int>(fminf(fmaxf(floorf(0.25f * (c[1] + c[3] + c[5] + c[7])), -most), most));
         sm.level[0] = a.levels ? a.levels[2 * qi] : 0.0f;
         sm.level[1] = a.levels ? a.levels[2 * qi + 1] : 255.0f;
+        sm.far = 0;
     }
     if (tid < 8) sm.c[tid] = corners[8 * qi + tid];
     load_grid(a, qi, sm.grid);
@@ -750,20 +751,21 @@ __global__ void __launch_bounds__(kGnWarps * 32, 2) k_refine_gauss_newton(bd_ref
                 if (lane < 8) {
                     const double ww = sm.sum[kWW + lane];
                     sm.wr[lane] = sm.sum[kWR + lane] - sm.shift[1] * ww - sm.shift[0] * (sm.sum[kWAll + lane] - ww);
-                } else if (lane == 8) {
-                    // A correction above the squared residuals would more than double the
-                    // rounding of their sum.  Below 2.5e-4 a level it is
-                    // lost in that of the values.  Some first steps exceed it: 6 us of 131.
-                    double moved = 0.0, left = 0.0;
-                    bool far = false;
-                    for (int i = 0; i < 2; ++i) {
-                        const double sh = sm.shift[i], n = sm.sum[kCount + i];
-                        moved += sh * sh * n;
-                        left += sm.sum[kMoment2 + i] - sh * (2.0 * sm.sum[kMoment1 + i] - sh * n);
-                        far = far || fabs(sh) > 2.5e-4;
-                    }
-                    sm.far = far && moved > left ? 1 : 0;
                 }
+            } else if (tid == 96 && !a.levels) {
+                // A correction above the squared residuals would more than double the
+                // rounding of their sum.  Below 2.5e-4 a level it is lost in that of
+                // the values.  In FP32 and by a warp of its own, beside the others' FP64: 6 us of 124 where not.
+                float moved = 0.0f, left = 0.0f;
+                bool far = false;
+                for (int i = 0; i < 2; ++i) {
+                    const float n = sm.sum[kCount + i], m1 = sm.sum[kMoment1 + i];
+                    const float sh = n > 0.0f ? m1 / n : 0.0f;
+                    moved += sh * m1;
+                    left += sm.sum[kMoment2 + i] - sh * m1;
+                    far = far || fabsf(sh) > 2.5e-4f;
+                }
+                sm.far = far && moved > left ? 1 : 0;
             }
             __syncthreads();
             if (!first_pass || !sm.far) break;

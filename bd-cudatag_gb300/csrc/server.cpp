@@ -372,8 +372,9 @@ int64_t bd_server_submit(bd_server* s, int32_t camera, const uint8_t* gray, int3
     }
     const auto arrival = Clock::now();
     cudaPointerAttributes attr;
-    const bool pinned = cudaPointerGetAttributes(&attr, gray) == cudaSuccess &&
-                        attr.type == cudaMemoryTypeHost;
+    const bool known = cudaPointerGetAttributes(&attr, gray) == cudaSuccess;
+    const bool pinned = known && attr.type == cudaMemoryTypeHost;
+    const bool on_device = known && attr.type == cudaMemoryTypeDevice;  // the CPU cannot copy it
     cudaGetLastError();
     std::unique_lock<std::mutex> lock(s->mutex);
     if (s->outstanding[camera] >= s->queue_depth || (!pinned && s->free_buffers[camera].empty())) {
@@ -395,25 +396,27 @@ int64_t bd_server_submit(bd_server* s, int32_t camera, const uint8_t* gray, int3
         const RequestBuffer& b = *r.owned;
         const bool strided = stride != cam.width;
         bool direct = b.device && !s->free_streams.empty() &&
-                            bdgb::copies_direct(stride, cam.width, cam.height) &&
-                            !(strided && s->strided_copies >= kStridedCopies);
+                      bdgb::copies_direct(stride, cam.width, cam.height) &&
+                      !(strided && s->strided_copies >= kStridedCopies);
         cudaStream_t stream = nullptr;
         if (direct) {
             stream = s->free_streams.back();
             s->free_streams.pop_back();
             if (strided) ++s->strided_copies;
         }
+        uint8_t* const to = direct || (on_device && b.device) ? b.device : b.pinned;
         lock.unlock();
         cudaError_t copied = cudaSuccess;
-        if (direct) {
+        if (direct || on_device) {
             bool refused = false;
-            copied = bdgb::copy_pageable(b.device, gray, stride, cam.width, cam.height, stream, &refused);
-            if (refused) {
+            copied = bdgb::copy_pageable(to, gray, stride, cam.width, cam.height,
+                                         stream ? stream : cudaStreamPerThread, &refused);
+            if (refused && !on_device) {
                 direct = false;
                 copied = cudaSuccess;
             }
         }
-        if (!direct) {
+        if (!direct && !on_device) {
             for (int y = 0; y < cam.height; ++y) {
                 std::memcpy(b.pinned + static_cast<size_t>(y) * cam.width,
                             gray + static_cast<size_t>(y) * stride, cam.width);
@@ -430,7 +433,7 @@ int64_t bd_server_submit(bd_server* s, int32_t camera, const uint8_t* gray, int3
             bdgb::set_last_error(cudaGetErrorString(copied));
             return BD_ERROR_CUDA;
         }
-        r.frame = direct ? b.device : b.pinned;
+        r.frame = direct || on_device ? to : b.pinned;
         r.stride = cam.width;
     }
     const int64_t ticket = s->next_ticket++;

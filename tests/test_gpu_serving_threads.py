@@ -18,6 +18,31 @@ SIZES = [(160, 120), (640, 480), (1283, 820), (1920, 1080)]  # below and above 1
 ROUNDS = 6
 
 
+@pytest.mark.parametrize("room", [False, True])
+@pytest.mark.parametrize("pad", [0, 7])
+def test_frames_in_device_memory(pad, room):
+    """Copied at submit like pageable ones, whatever way those of the same shape take."""
+    cameras = [(w, h, 1) for w, h in SIZES]
+    plan = bdcudatag.Batch(cameras).device_bytes()
+    server = bdcudatag.Server(cameras, device_budget=plan + (64 << 20 if room else 0), max_batches=1, queue_depth=12)
+    tickets = []
+    for c, (w, h) in enumerate(SIZES):
+        frame = scenes.ref_scenes(w, h, 1)[0][0]
+        rows = torch.full((h, w + pad), 255, dtype=torch.uint8, device="cuda")
+        rows[:, :w] = torch.from_numpy(np.ascontiguousarray(frame)).cuda()
+        torch.cuda.synchronize()
+        tickets.append((server.submit(c, rows, w + pad), frame))
+        assert tickets[-1][0] >= 0, bdcudatag.last_error()
+        rows.zero_()
+        torch.cuda.synchronize()
+    for ticket, frame in tickets:
+        rc, found, out, _ = server.wait(ticket)
+        n, records = oracle.Frame(np.ascontiguousarray(frame), 0).detections()
+        assert rc == 1 and found[0] == n
+        same_records(out[0, :n], records)
+    server.close()
+
+
 @pytest.mark.parametrize("room", [False, True])  # request buffers in host memory, in device memory
 def test_threads(room):
     cameras = [(w, h, 1) for w, h in SIZES]

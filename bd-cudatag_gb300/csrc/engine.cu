@@ -89,20 +89,40 @@ bool device_reads_pageable(int device) {
     return access != 0 && tables != 0;
 }
 
+namespace {
+
+// A capture that another thread has open in the global mode does not concern the
+// streams that pageable frames are copied on.
+class RelaxedCapture {
+public:
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode_); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode_); }
+    RelaxedCapture(const RelaxedCapture&) = delete;
+    RelaxedCapture& operator=(const RelaxedCapture&) = delete;
+
+private:
+    cudaStreamCaptureMode mode_ = cudaStreamCaptureModeRelaxed;
+};
+
+// False where the runtime does not take the copy; nothing happened then.
+bool queue_pageable(uint8_t* dst, const uint8_t* src, int stride, int width, int height, cudaStream_t stream,
+                    cudaError_t* error) {
+    *error = stride == width
+                 ? cudaMemcpyAsync(dst, src, static_cast<size_t>(width) * height, cudaMemcpyDefault, stream)
+                 : cudaMemcpy2DAsync(dst, width, src, stride, width, height, cudaMemcpyDefault, stream);
+    if (*error == cudaSuccess) return true;
+    cudaGetLastError();
+    return false;
+}
+
+}  // namespace
+
 cudaError_t copy_pageable(uint8_t* dst, const uint8_t* src, int stride, int width, int height,
                           cudaStream_t stream, bool* refused) {
-    // A capture that another thread has open in the global mode does not concern this stream.
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    cudaThreadExchangeStreamCaptureMode(&mode);
-    const cudaError_t queued =
-        stride == width
-            ? cudaMemcpyAsync(dst, src, static_cast<size_t>(width) * height, cudaMemcpyDefault, stream)
-            : cudaMemcpy2DAsync(dst, width, src, stride, width, height, cudaMemcpyDefault, stream);
-    *refused = queued != cudaSuccess;
-    if (*refused) cudaGetLastError();
-    const cudaError_t done = *refused ? queued : cudaStreamSynchronize(stream);
-    cudaThreadExchangeStreamCaptureMode(&mode);
-    return done;
+    const RelaxedCapture relaxed;
+    cudaError_t error;
+    *refused = !queue_pageable(dst, src, stride, width, height, stream, &error);
+    return *refused ? error : cudaStreamSynchronize(stream);
 }
 
 // The plan's device made current while a call launches kernels or sets their
@@ -546,12 +566,30 @@ int Plan::submit_host(const uint8_t* const* frames, const int32_t* strides, std:
     // staging buffer (the reference's detect_host path, gpu_detector.cu:2169-2176),
     // as is any pageable frame under a stream capture, whose replays read it there (a
     // plan without graphs; one with graphs refuses to be captured).
+    //
+    // A copy costs the call some 9 us, and the memcpy of a frame as much at 150 KB.  A
+    // frame alone gains at any size all the same (its wait replaces the copy in the graph: 27 KB 91 ->
+    // 86 us a call, 300 KB 116 -> 97), one of several from 200 KB on (sixteen frames
+    // of 320x240 200 us staged and 270 direct, 512x384 287 and 296, 576x432 327 and 302).
+    const size_t tight_from = this->frames() == 1 ? 0 : 200 << 10;
     enum : uint8_t { kStaged, kPinned, kPageable };
     uint8_t source[kMaxFrames] = {};
     bool any_direct = false;
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     if (im.reads_pageable && s != im.stream) cudaStreamIsCapturing(s, &capture);
     const bool pageable = im.reads_pageable && capture == cudaStreamCaptureStatusNone;
+    auto stage = [&](int i) {
+        const int w = frames_[i].width, h = frames_[i].height;
+        uint8_t* dst = im.frames_pinned + im.frame_offset[i];
+        if (strides[i] == w) {
+            std::memcpy(dst, frames[i], static_cast<size_t>(w) * h);
+        } else {
+            for (int y = 0; y < h; ++y) {
+                std::memcpy(dst + static_cast<size_t>(y) * w,
+                            frames[i] + static_cast<size_t>(y) * strides[i], w);
+            }
+        }
+    };
     for (int i = 0; i < this->frames(); ++i) {
         if (!frames[i]) {
             if (error) *error = "null image pointer";
@@ -567,46 +605,40 @@ int Plan::submit_host(const uint8_t* const* frames, const int32_t* strides, std:
             // not this submit's.
             cudaGetLastError();
             if (known && attr.type == cudaMemoryTypeUnregistered && pageable &&
-                copies_direct(strides[i], frames_[i].width, frames_[i].height)) {
+                copies_direct(strides[i], frames_[i].width, frames_[i].height, tight_from)) {
                 source[i] = kPageable;
+            } else {
+                // Here and not in a loop of its own: with the query between one frame and the
+                // next, memcpy moves 26 GB/s, frame after frame 18.
+                stage(i);
             }
         }
         any_direct = any_direct || source[i] != kStaged;
-    }
-    auto stage = [&](int i) {
-        const int w = frames_[i].width, h = frames_[i].height;
-        uint8_t* dst = im.frames_pinned + im.frame_offset[i];
-        if (frames[i] == dst) return;
-        if (strides[i] == w) {
-            std::memcpy(dst, frames[i], static_cast<size_t>(w) * h);
-        } else {
-            for (int y = 0; y < h; ++y) {
-                std::memcpy(dst + static_cast<size_t>(y) * w,
-                            frames[i] + static_cast<size_t>(y) * strides[i], w);
-            }
-        }
-    };
-    for (int i = 0; i < this->frames(); ++i) {
-        if (source[i] == kStaged) stage(i);
     }
     // The batch's GPU time has the copies to the device in it, not the CPU's.
     cudaEventRecord(im.ev_start, s);
     // The pageable ones on the plan's own stream, which is idle here: the call
     // waits for them, and not for what the caller's stream still has to do.  One that
     // the runtime does not take goes through the staging buffer.
+    // All are queued before the one wait, which takes 8 us or so.
     if (any_direct) {
+        const RelaxedCapture relaxed;
+        bool queued = false;
         for (int i = 0; i < this->frames(); ++i) {
             if (source[i] != kPageable) continue;
-            bool refused = false;
-            const cudaError_t st = copy_pageable(im.frames_dev + im.frame_offset[i], frames[i], strides[i],
-                                                 frames_[i].width, frames_[i].height, im.stream, &refused);
-            if (refused) {
+            cudaError_t st;
+            if (queue_pageable(im.frames_dev + im.frame_offset[i], frames[i], strides[i], frames_[i].width,
+                               frames_[i].height, im.stream, &st)) {
+                queued = true;
+            } else {
                 source[i] = kStaged;
                 stage(i);
-            } else if (st != cudaSuccess) {
-                if (error) *error = cuda_error("cudaMemcpyAsync(frame)", st);
-                return -1;
             }
+        }
+        const cudaError_t st = queued ? cudaStreamSynchronize(im.stream) : cudaSuccess;
+        if (st != cudaSuccess) {
+            if (error) *error = cuda_error("cudaMemcpyAsync(frame)", st);
+            return -1;
         }
     }
     if (!any_direct) {

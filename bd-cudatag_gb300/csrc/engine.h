@@ -44,11 +44,12 @@ int auto_max_candidates(int width, int height, int configured);
 // that its copy engine takes it as fast as page-locked memory.
 bool device_reads_pageable(int device);
 
-// Whether a pageable frame of rows `stride` bytes apart goes that way.  Rows with a
+// Whether a pageable frame of rows `stride` bytes apart goes that way, `tight_from` bytes
+// being the least for one without a gap between its rows.  Rows with a
 // gap are copied row by row, on which a small frame loses (300 KB: 28 us against 21
 // through page-locked memory; 1 MB: 47 to 72 against 74; 8 MB: 134 against 644).
-inline bool copies_direct(int stride, int width, int height) {
-    return stride == width || static_cast<size_t>(width) * height >= size_t{1} << 20;
+inline bool copies_direct(int stride, int width, int height, size_t tight_from) {
+    return static_cast<size_t>(width) * height >= (stride == width ? tight_from : size_t{1} << 20);
 }
 
 // Copies a pageable frame to tight rows in device memory, on a device that

@@ -34,7 +34,7 @@ thread_local cudaError_t t_error = cudaSuccess;
 thread_local Graph* t_capture = nullptr;
 std::mutex g_mutex;
 std::map<const char*, std::pair<size_t, cudaMemoryType>> g_memory;
-std::atomic<int> g_launches{0}, g_updates{0}, g_refuse{0}, g_slow{0}, g_staged{0}, g_live_streams{0};
+std::atomic<int> g_launches{0}, g_updates{0}, g_refuse{0}, g_slow{0}, g_staged{0}, g_direct{0}, g_waits{0}, g_live_streams{0};
 
 cudaError_t fail(cudaError_t e) { return t_error = e; }
 Stream* stream_of(cudaStream_t s) { return reinterpret_cast<Stream*>(s); }
@@ -64,6 +64,7 @@ cudaMemoryType type_of(const void* p) {
 cudaError_t copy(void* dst, size_t dpitch, const void* src, size_t spitch, size_t width, size_t height, cudaStream_t s) {
     if (type_of(src) == cudaMemoryTypeUnregistered) {
         if (g_refuse) return fail(cudaErrorInvalidValue);
+        ++g_direct;
         const int first = *static_cast<const unsigned char*>(src);
         std::lock_guard<std::mutex> lock(g_mutex);
         Stream* st = stream_of(s);
@@ -96,6 +97,8 @@ extern "C" {
 int fake_launches() { return g_launches; }
 int fake_updates() { return g_updates; }
 int fake_copies_from_page_locked() { return g_staged; }
+int fake_direct_copies() { return g_direct; }
+int fake_waits() { return g_waits; }
 int fake_streams() { return g_live_streams; }
 void fake_refuse(int on) { g_refuse = on; }
 void fake_slow(int ms) { g_slow = ms; }
@@ -140,6 +143,7 @@ cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) {
 cudaError_t cudaStreamDestroy(cudaStream_t s) { --g_live_streams; delete stream_of(s); return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t s) {
     if (!s) return cudaSuccess;
+    ++g_waits;
     for (;;) {
         Clock::time_point until;
         {

@@ -138,3 +138,20 @@ def test_errors_of_earlier_calls(stand_in):
             assert L.cudaSetDevice(99) != 0
             batch.detect(frames)
     """)
+
+
+def test_pageable_frames_of_a_batch(stand_in):
+    """Several pageable frames: small ones are staged, larger ones are all queued before
+    one wait; a frame alone is copied direct at any size."""
+    run(stand_in, """
+        for size, count, direct in ((64, 1, 1), (320, 16, 0), (1024, 5, 5)):
+            batch = bdcudatag.Batch([(size, size * 3 // 4, 1)] * count)
+            copies, waits = L.fake_direct_copies(), L.fake_waits()
+            batch.detect([frame(size, size * 3 // 4) for _ in range(count)])
+            assert L.fake_direct_copies() - copies == direct
+            assert L.fake_waits() - waits == min(direct, 1)
+        mixed = bdcudatag.Batch([(160, 120, 1), (1024, 768, 1)])
+        copies = L.fake_direct_copies()
+        mixed.detect([frame(160, 120), frame(1024, 768)])
+        assert L.fake_direct_copies() - copies == 1
+    """)

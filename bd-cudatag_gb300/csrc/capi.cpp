@@ -248,7 +248,8 @@ bd_detector* bd_detector_create(int32_t family, int32_t width, int32_t height,
         if (status_out) *status_out = BD_ERROR_INVALID_ARGUMENT;
         return nullptr;
     }
-    const bdgb::PlanConfig pc = bdgb::resolve_config(config);
+    bdgb::PlanConfig pc = bdgb::resolve_config(config);
+    pc.one_at_a_time = true;
     bdgb::PlanFrame frame;
     frame.width = width;
     frame.height = height;

@@ -456,6 +456,7 @@ Plan* Plan::create(const std::vector<PlanFrame>& frames, const PlanConfig& confi
     hd.band_prefix[nf] = bands;
     hd.total_bands = bands;
     im.launch_cfg = default_launch(hd, im.sm_count);
+    im.launch_cfg.one_at_a_time = config.one_at_a_time;
     set_stats_rows(hd, im.launch_cfg.stats_rows);
     plan->arena_bytes_ = carve.off;
 
@@ -775,6 +776,7 @@ int Plan::set_launch(const LaunchConfig& lc, std::string* error) {
     if (im.pending && wait(error) != 0) return -1;
     cudaStreamSynchronize(im.stream);
     im.launch_cfg = lc;
+    im.launch_cfg.one_at_a_time = config_.one_at_a_time;
     set_stats_rows(im.host_desc, lc.stats_rows);
     const cudaError_t st = cudaMemcpy(im.dev_desc, &im.host_desc, sizeof(BatchDesc),
                                       cudaMemcpyHostToDevice);

@@ -32,6 +32,7 @@ struct PlanConfig {
     int max_candidates = 0;       // 0: per frame, from the frame area
     bool refine_edges = true;
     bool use_graph = true;
+    bool one_at_a_time = false;   // every batch is waited for before the next (a detector)
     float min_decision_margin = 3.0f;
     float decode_sharpening = 0.25f;
 };

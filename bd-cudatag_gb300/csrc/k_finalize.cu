@@ -85,7 +85,8 @@ void enqueue_pipeline(const BatchDesc* dd, const BatchDesc& hd, const FrameIOArg
     // of 256 threads, and a batch of few such bands (two per SM at most) leaves the GPU
     // idle besides: a noisy 3840x2160 frame takes 62 us instead of 79 in
     // k_binarize_runs with two warps per row, and 25 instead of 31 in k_cand_count
-    // with 512 threads.  k_merge takes 512 only beyond 4096 pixels: in flight its larger
+    // with 512 threads.  k_merge takes 512 beyond 4096 pixels and for detectors, which have
+    // one frame at a time: in flight its larger
     // CTAs cost more than they give alone (noise, alone and seven or so in flight: 3840x2160 126 and 455 us
     // with 512 in k_merge, 132 and 386 with 256; 5120x2400 149 and 410, 159 and 369; 8192x2400
     // 217 and 452, 277 and 480 with 256 in all).
@@ -100,7 +101,7 @@ void enqueue_pipeline(const BatchDesc* dd, const BatchDesc& hd, const FrameIOArg
     const bool more = few_bands && words_max > 96;  // wider than 3072 pixels
     const int row_warps = more ? 2 : 1;
     const int run_threads = more ? 512 : (!few_bands && words_max <= 64 ? 128 : 256);
-    const int merge_threads = more && words_max <= 128 ? 256 : run_threads;
+    const int merge_threads = more && words_max <= 128 && !lc.one_at_a_time ? 256 : run_threads;
     const BinarizeKernel binarize = binarize_kernel(row_warps);
     binarize<<<bands, 256 * row_warps, band_smem_bytes(lc.band_cap, words_max), s>>>(dd, io, lc.band_cap,
                                                                                       words_max);

@@ -171,6 +171,7 @@ struct LaunchConfig {
     int fit_merged = 0;        // 1: big and small candidates in one fit-and-decode launch
     int persistent = 0;        // 1: the whole batch as one persistent launch (k_persistent.cu)
     int persist_ctas = 0;      // CTAs of that launch (0: every SM's resident maximum)
+    bool one_at_a_time = false;  // the plan's (PlanConfig), not tuned
 };
 
 // A second stream and two events for the parallel branch of the pipeline

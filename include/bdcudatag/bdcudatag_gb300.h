@@ -160,7 +160,7 @@ BD_API int32_t bd_batch_pipeline(bd_batch* const* batches, int32_t count,
  * passing this pointer as frames[i]. */
 BD_API uint8_t* bd_batch_host_frame(bd_batch* batch, int32_t camera);
 
-/* GPU time of the last completed batch (events around the graph), ms. */
+/* GPU time of the last completed batch, from its first copy to the device on, ms. */
 BD_API float bd_batch_last_gpu_ms(const bd_batch* batch);
 
 /* Pipeline counters of camera i in the last batch: [0] candidates before

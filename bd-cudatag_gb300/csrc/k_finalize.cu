@@ -26,7 +26,7 @@ int prepare_pipeline() {
         }
     }
     if (cudaFuncSetAttribute(k_cand_count, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(cand_smem_bytes(kMaxBandsPerFrame, kMaxBandsPerFrame))) != cudaSuccess) {
+                             static_cast<int>(cand_smem_bytes(kMaxBandsPerFrame, kTableBands))) != cudaSuccess) {
         return -1;
     }
     if (cudaFuncSetAttribute(k_fit_decode_all, cudaFuncAttributeMaxDynamicSharedMemorySize,

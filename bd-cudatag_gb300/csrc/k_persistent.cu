@@ -303,7 +303,7 @@ size_t persistent_smem_bytes(int band_cap, int bits_words, int row_cap_max, size
 int prepare_persistent() {
     // The largest overlay: band cap 2048 on the widest frame, tallest frame.
     const size_t most = persistent_smem_bytes(kMaxBandCap, BD_MAX_WIDTH / 32, BD_MAX_WIDTH / 2 + 2,
-                                              cand_smem_bytes(kMaxBandsPerFrame, kMaxBandsPerFrame));
+                                              cand_smem_bytes(kMaxBandsPerFrame, kTableBands));
     return cudaFuncSetAttribute(k_persistent, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 static_cast<int>(most)) == cudaSuccess
                ? 0
